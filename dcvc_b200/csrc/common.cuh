@@ -51,6 +51,21 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p)
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// 16 bytes of shared memory by address: pointers into the aligned dynamic buffer are generic to the
+// compiler.
+__device__ __forceinline__ uint4 lds128(uint32_t addr)
+{
+    uint4 v;
+    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
+    return v;
+}
+
+__device__ __forceinline__ void sts128(uint32_t addr, uint4 v)
+{
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
+                 : "memory");
+}
+
 // ---------------------------------------------------------------- mbarrier (bounded waits)
 
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count)
@@ -105,6 +120,53 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
     return true;
 }
 
+// The same for a barrier that also receives arrivals from the other CTA of a pair: acquires at
+// cluster scope.
+__device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t parity)
+{
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+
+// mbar_wait_bounded by a whole converged warp with one answer for all lanes.  The warps that feed
+// the tensor cores and the copy engine run their loops on all 32 lanes and let one elected lane
+// issue: with the loop inside `if (lane == 0)` a stage of four MMAs costs its issuer 565 clocks
+// whatever their width, with uniform control flow 400 (measured with everything else in place
+// taken away), and four 256-wide MMAs run for 512.
+template <bool CLUSTER = false>
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, long long limit_cycles)
+{
+    auto ready = [&] { return CLUSTER ? mbar_try_wait_cluster(bar, parity) : mbar_try_wait(bar, parity); };
+    if (__all_sync(0xffffffffu, ready())) {
+        return true;
+    }
+    const long long t0 = clock64();
+    while (!__all_sync(0xffffffffu, ready())) {
+        if (__any_sync(0xffffffffu, clock64() - t0 > limit_cycles)) {
+            return false;
+        }
+    }
+    return true;
+}
+
+// One answer for a whole converged warp.
+__device__ __forceinline__ bool warp_any(bool b) { return __any_sync(0xffffffffu, b); }
+
+// True in one lane of a converged warp (always the same one).
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+
 // ---------------------------------------------------------------- TMA
 
 __device__ __forceinline__ void tma_prefetch_desc(const void* tmap)
@@ -121,6 +183,15 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const void* tmap, uint64_
         " [%0], [%1, {%3, %4}], [%2];" ::"r"(smem_u32(dst)),
         "l"(reinterpret_cast<uint64_t>(tmap)), "r"(smem_u32(bar)), "r"(c0), "r"(c1)
         : "memory");
+}
+
+// Brings a tile of a 2D tensor into L2.
+__device__ __forceinline__ void tma_prefetch_2d(const void* tmap, int c0, int c1)
+{
+    asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];" ::"l"(
+                     reinterpret_cast<uint64_t>(tmap)),
+                 "r"(c0), "r"(c1)
+                 : "memory");
 }
 
 // 2D tiled store from shared memory (bulk-group completion), no multicast.
@@ -236,6 +307,16 @@ __device__ __forceinline__ void tmem_ld_32x32b_x32(uint32_t taddr, uint32_t (&r)
         : "r"(taddr));
 }
 
+// Four consecutive 32-bit columns of this warp's 32 lanes (thread t writes lane base + t).
+__device__ __forceinline__ void tmem_st_32x32b_x4(uint32_t taddr, const uint32_t (&r)[4])
+{
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(taddr), "r"(r[0]), "r"(r[1]),
+                 "r"(r[2]), "r"(r[3])
+                 : "memory");
+}
+
+__device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
 // Shared-memory matrix descriptor for a K-major operand tile written by TMA with 128-byte
 // swizzle: rows of 64 16-bit elements (128 B), 8-row groups 1024 B apart.
 DCVC_HOST_DEVICE uint64_t make_sw128_kmajor_desc(uint32_t smem_addr)
@@ -293,7 +374,18 @@ __device__ __forceinline__ uint32_t cluster_map(const void* p, uint32_t rank)
 // Arrive on an mbarrier of another CTA of the cluster (address from cluster_map).
 __device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr)
 {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+
+// `n` arrivals at once, on this CTA's barrier or on another CTA's.
+__device__ __forceinline__ void mbar_arrive_n(uint64_t* bar, uint32_t n)
+{
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(n) : "memory");
+}
+
+__device__ __forceinline__ void mbar_arrive_remote_n(uint32_t cluster_addr, uint32_t n)
+{
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0], %1;" ::"r"(cluster_addr), "r"(n) : "memory");
 }
 
 // 2D tiled load into this CTA's shared memory whose completion is counted on a barrier of the
@@ -333,6 +425,19 @@ __device__ __forceinline__ void tc_mma_f16_pair(uint32_t tmem_d, uint64_t adesc,
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
         "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+
+// The same with A in tensor memory: each CTA's 128 rows in its lanes, 16-bit K elements packed two
+// to a column.
+__device__ __forceinline__ void tc_mma_f16_pair_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
+                                                   uint32_t accumulate)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
+        "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
 

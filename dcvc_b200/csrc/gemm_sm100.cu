@@ -202,36 +202,48 @@ __global__ void __launch_bounds__(GemmCfg<BN, EPI, PAIR>::kThreads, 1)
     griddep_launch_dependents();
     griddep_wait();
 
+    // The producer and the MMA warp run their loops on all lanes (see mbar_wait_warp); one elected
+    // lane issues the copies and the MMAs.
+    auto fail = [&](int code) {
+        *abort_flag = 1;
+        if (lane == 0) {
+            report_error(p.err, code);
+        }
+        return false;
+    };
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
-        if (lane == 0 && !p.stall_test) {
+        if (!p.stall_test) {
             int stage = 0;
             uint32_t phase = 0;
             int issued = 0;
-            for (int tile = unit; tile < num_tiles && !*abort_flag; tile += units) {
+            bool ok = true;
+            for (int tile = unit; ok && tile < num_tiles && !warp_any(*abort_flag != 0); tile += units) {
                 const int m0 = (tile % num_m) * kTileM + row_off;
                 const int n0 = (tile / num_m) * BN;
                 for (int kb = 0; kb < kblocks; ++kb) {
-                    if (!mbar_wait_bounded(&empty[stage], phase ^ 1, lim)) {
-                        *abort_flag = 1;
-                        report_error(p.err, kErrGemmProducerTimeout);
+                    if (!mbar_wait_warp(&empty[stage], phase ^ 1, lim)) {
+                        ok = fail(kErrGemmProducerTimeout);
                         break;
                     }
-                    uint8_t* sa = smem + stage * C::kStageBytes;
-                    if constexpr (PAIR) {
-                        // the even CTA's barrier counts both CTAs' bytes
-                        if (rank == 0) {
-                            mbar_arrive_expect_tx(&full[stage], 2 * C::kStageBytes);
+                    if (elect_one()) {
+                        uint8_t* sa = smem + stage * C::kStageBytes;
+                        if constexpr (PAIR) {
+                            // the even CTA's barrier counts both CTAs' bytes
+                            if (rank == 0) {
+                                mbar_arrive_expect_tx(&full[stage], 2 * C::kStageBytes);
+                            }
+                            const uint32_t fb = cluster_map(&full[stage], 0);
+                            tma_load_2d_pair(sa, &tmA, fb, kb * kKElems, m0);
+                            tma_load_2d_pair(sa + C::kABytes, &tmB, fb, kb * kKElems,
+                                             n0 + static_cast<int>(rank) * (BN / 2));
+                        } else {
+                            mbar_arrive_expect_tx(&full[stage], C::kStageBytes);
+                            tma_load_2d(sa, &tmA, &full[stage], kb * kKElems, m0);
+                            tma_load_2d(sa + C::kABytes, &tmB, &full[stage], kb * kKElems, n0);
                         }
-                        const uint32_t fb = cluster_map(&full[stage], 0);
-                        tma_load_2d_pair(sa, &tmA, fb, kb * kKElems, m0);
-                        tma_load_2d_pair(sa + C::kABytes, &tmB, fb, kb * kKElems,
-                                         n0 + static_cast<int>(rank) * (BN / 2));
-                    } else {
-                        mbar_arrive_expect_tx(&full[stage], C::kStageBytes);
-                        tma_load_2d(sa, &tmA, &full[stage], kb * kKElems, m0);
-                        tma_load_2d(sa + C::kABytes, &tmB, &full[stage], kb * kKElems, n0);
                     }
+                    __syncwarp();
                     ++issued;
                     if (++stage == kStages) {
                         stage = 0;
@@ -239,8 +251,8 @@ __global__ void __launch_bounds__(GemmCfg<BN, EPI, PAIR>::kThreads, 1)
                     }
                 }
             }
-            if (*abort_flag && (!PAIR || rank == 0)) {
-                // Let the copies this thread issued land before the CTA winds down (PAIR: the
+            if (warp_any(*abort_flag != 0) && (!PAIR || rank == 0)) {
+                // Let the copies this warp issued land before the CTA winds down (PAIR: the
                 // even CTA's barriers count the peer's copies too; the odd CTA cannot observe its
                 // own copies, so after an abort it relies on the even CTA's drain, which waits
                 // (bounded) for both CTAs' bytes of each stage it issued, and on the cluster
@@ -252,82 +264,88 @@ __global__ void __launch_bounds__(GemmCfg<BN, EPI, PAIR>::kThreads, 1)
                         stage = kStages - 1;
                         phase ^= 1;
                     }
-                    mbar_wait_bounded(&full[stage], phase, kWaitLimit / 16);
+                    mbar_wait_warp(&full[stage], phase, kWaitLimit / 16);
                 }
             }
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
-        if (lane == 0 && (!PAIR || rank == 0)) {
+        if (!PAIR || rank == 0) {
             // format 0 is F16 for kind::f16 and E4M3 for kind::f8f6f4
             const uint32_t idesc = make_idesc_f16(kTileM, BN, F8 ? 0 : Pack2<T>::kFormat);
+            const uint32_t smem_addr = smem_u32(smem);
             int stage = 0;
             uint32_t phase = 0;
             int acc = 0;
             uint32_t acc_phase = 0;
             bool issued_any = false;
-            for (int tile = unit; tile < num_tiles && !*abort_flag; tile += units) {
-                if (!mbar_wait_bounded(&tempty[acc], acc_phase ^ 1, lim)) {
-                    *abort_flag = 1;
-                    report_error(p.err, kErrGemmMmaTimeout);
+            bool ok = true;
+            for (int tile = unit; ok && tile < num_tiles && !warp_any(*abort_flag != 0); tile += units) {
+                if (!mbar_wait_warp(&tempty[acc], acc_phase ^ 1, lim)) {
+                    ok = fail(kErrGemmMmaTimeout);
                     break;
                 }
                 tc_fence_after();
                 const uint32_t d = tmem_base + static_cast<uint32_t>(acc * BN);
                 for (int kb = 0; kb < kblocks; ++kb) {
-                    if (!mbar_wait_bounded(&full[stage], phase, lim)) {
-                        *abort_flag = 1;
-                        report_error(p.err, kErrGemmMmaTimeout);
+                    if (!mbar_wait_warp(&full[stage], phase, lim)) {
+                        ok = fail(kErrGemmMmaTimeout);
                         break;
                     }
                     tc_fence_after();
-                    const uint8_t* sa = smem + stage * C::kStageBytes;
-                    const uint64_t adesc = make_sw128_kmajor_desc(smem_u32(sa));
-                    const uint64_t bdesc = make_sw128_kmajor_desc(smem_u32(sa + C::kABytes));
+                    if (elect_one()) {
+                        const uint32_t sa = smem_addr + stage * C::kStageBytes;
+                        const uint64_t adesc = make_sw128_kmajor_desc(sa);
+                        const uint64_t bdesc = make_sw128_kmajor_desc(sa + C::kABytes);
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        // +32 bytes per instruction inside the swizzle atom (descriptor units of
-                        // 16 B): K = 16 16-bit or K = 32 8-bit elements
-                        if constexpr (F8) {
-                            tc_mma_f8(d, adesc + 2 * k, bdesc + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
-                        } else if constexpr (PAIR) {
-                            tc_mma_f16_pair(d, adesc + 2 * k, bdesc + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
+                        for (int k = 0; k < 4; ++k) {
+                            // +32 bytes per instruction inside the swizzle atom (descriptor units of
+                            // 16 B): K = 16 16-bit or K = 32 8-bit elements
+                            if constexpr (F8) {
+                                tc_mma_f8(d, adesc + 2 * k, bdesc + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
+                            } else if constexpr (PAIR) {
+                                tc_mma_f16_pair(d, adesc + 2 * k, bdesc + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
+                            } else {
+                                tc_mma_f16(d, adesc + 2 * k, bdesc + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
+                            }
+                        }
+                        if constexpr (PAIR) {
+                            tc_commit_pair_both(&empty[stage]);  // frees the stage in both CTAs
                         } else {
-                            tc_mma_f16(d, adesc + 2 * k, bdesc + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
+                            tc_commit(&empty[stage]);
+                        }
+                        if (kb == kblocks - 1) {
+                            if constexpr (PAIR) {
+                                tc_commit_pair_both(&tfull[acc]);
+                            } else {
+                                tc_commit(&tfull[acc]);
+                            }
                         }
                     }
+                    __syncwarp();
                     issued_any = true;
-                    if constexpr (PAIR) {
-                        tc_commit_pair_both(&empty[stage]);  // frees the stage in both CTAs
-                    } else {
-                        tc_commit(&empty[stage]);
-                    }
                     if (++stage == kStages) {
                         stage = 0;
                         phase ^= 1;
                     }
-                }
-                if (*abort_flag) {
-                    break;
-                }
-                if constexpr (PAIR) {
-                    tc_commit_pair_both(&tfull[acc]);
-                } else {
-                    tc_commit(&tfull[acc]);
                 }
                 acc ^= 1;
                 if (acc == 0) {
                     acc_phase ^= 1;
                 }
             }
-            if (*abort_flag && issued_any) {
-                // Drain this thread's outstanding MMAs before the columns are released.
-                if constexpr (PAIR) {
-                    tc_commit_pair_local(drain);
-                } else {
-                    tc_commit(drain);
+            if (warp_any(*abort_flag != 0) && issued_any) {
+                // Drain this warp's outstanding MMAs before the columns are released (a commit
+                // tracks its own thread's MMAs: the elected lane is the same throughout).
+                if (elect_one()) {
+                    if constexpr (PAIR) {
+                        tc_commit_pair_local(drain);
+                    } else {
+                        tc_commit(drain);
+                    }
                 }
-                mbar_wait_bounded(drain, 0, kWaitLimit / 16);
+                __syncwarp();
+                mbar_wait_warp(drain, 0, kWaitLimit / 16);
             }
         }
     } else {

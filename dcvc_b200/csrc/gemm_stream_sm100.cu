@@ -27,7 +27,7 @@
 // each of the four channel slices recomputes the depthwise values of its rows, and with two band
 // sets in shared memory the producers wait for every band's L2 latency.  The codecs therefore use
 // it only when asked to (gemm_set_dw_fusion).
-// One thread issues tcgen05.mma (M = 128, N = 128, K = 16) into a double-buffered FP32 TMEM
+// One lane issues tcgen05.mma (M = 128, N = 128, K = 16) into a double-buffered FP32 TMEM
 // accumulator.  Per output element the products are summed in the same order as in the tiled
 // kernel and the epilogue applies bias, residual(s) and x q in the same order, so the outputs
 // are bitwise those of gemm_sm100 at any tile width.
@@ -219,6 +219,13 @@ __global__ void __launch_bounds__(StreamCfg<EPI, DW>::kThreads, 1)
     griddep_launch_dependents();
     griddep_wait();
 
+    auto fail = [&](int code) {
+        *abort_flag = 1;
+        if (lane == 0) {
+            report_error(p.err, code);
+        }
+        return false;
+    };
     if (DW && warp < C::kProdWarps) {
         // ------------------------------------------------------------ depthwise producers
         // Step v fills half `v & 1` (64 rows) of the A stage of unit u = v >> 1 = (tile
@@ -377,25 +384,32 @@ __global__ void __launch_bounds__(StreamCfg<EPI, DW>::kThreads, 1)
         }
     } else if (!DW && warp == 0) {
         // ------------------------------------------------------------ TMA producer
-        if (lane == 0 && ntiles > 0 && !p.stall_test) {
+        // (all lanes run the loops of this and the MMA warp, one elected lane issues: see mbar_wait_warp)
+        if (ntiles > 0 && !p.stall_test) {
             // the W slice once: kblocks boxes of 128 rows x 64 K
-            mbar_arrive_expect_tx(bfull, static_cast<uint32_t>(kblocks * kSBN * kSBK * 2));
-            for (int kb = 0; kb < kblocks; ++kb) {
-                tma_load_2d(smem + C::kBOffset + kb * kSBN * 128, &tmB, bfull, kb * kSBK, n0);
+            if (elect_one()) {
+                mbar_arrive_expect_tx(bfull, static_cast<uint32_t>(kblocks * kSBN * kSBK * 2));
+                for (int kb = 0; kb < kblocks; ++kb) {
+                    tma_load_2d(smem + C::kBOffset + kb * kSBN * 128, &tmB, bfull, kb * kSBK, n0);
+                }
             }
+            __syncwarp();
             int stage = 0;
             uint32_t phase = 0;
             int issued = 0;
-            for (int t = 0; t < ntiles && !*abort_flag; ++t) {
+            bool ok = true;
+            for (int t = 0; ok && t < ntiles && !warp_any(*abort_flag != 0); ++t) {
                 const int m0 = r0 + t * kSBM;
                 for (int kb = 0; kb < kblocks; ++kb) {
-                    if (!mbar_wait_bounded(&empty[stage], phase ^ 1, lim)) {
-                        *abort_flag = 1;
-                        report_error(p.err, kErrGemmProducerTimeout);
+                    if (!mbar_wait_warp(&empty[stage], phase ^ 1, lim)) {
+                        ok = fail(kErrGemmProducerTimeout);
                         break;
                     }
-                    mbar_arrive_expect_tx(&full[stage], kSABytes);
-                    tma_load_2d(smem + C::kAOffset + stage * kSABytes, &tmA, &full[stage], kb * kSBK, m0);
+                    if (elect_one()) {
+                        mbar_arrive_expect_tx(&full[stage], kSABytes);
+                        tma_load_2d(smem + C::kAOffset + stage * kSABytes, &tmA, &full[stage], kb * kSBK, m0);
+                    }
+                    __syncwarp();
                     ++issued;
                     if (++stage == kStages) {
                         stage = 0;
@@ -403,75 +417,74 @@ __global__ void __launch_bounds__(StreamCfg<EPI, DW>::kThreads, 1)
                     }
                 }
             }
-            if (*abort_flag) {
-                // let this thread's copies land before the CTA winds down
-                mbar_wait_bounded(bfull, 0, kSWaitLimit / 16);
+            if (warp_any(*abort_flag != 0)) {
+                // let this warp's copies land before the CTA winds down
+                mbar_wait_warp(bfull, 0, kSWaitLimit / 16);
                 int n = issued < kStages ? issued : kStages;
                 for (int i = 0; i < n; ++i) {
                     if (--stage < 0) {
                         stage = kStages - 1;
                         phase ^= 1;
                     }
-                    mbar_wait_bounded(&full[stage], phase, kSWaitLimit / 16);
+                    mbar_wait_warp(&full[stage], phase, kSWaitLimit / 16);
                 }
             }
         }
     } else if (warp == C::kMmaWarp) {
         // ------------------------------------------------------------ MMA issuer
-        if (lane == 0 && ntiles > 0) {
+        if (ntiles > 0) {
             const uint32_t idesc = make_idesc_f16(kSBM, kSBN, SPack2<T>::kFormat);
+            const uint32_t smem_addr = smem_u32(smem);
             int stage = 0;
             uint32_t phase = 0;
             int acc = 0;
             uint32_t acc_phase = 0;
             bool issued_any = false;
-            if (!mbar_wait_bounded(bfull, 0, lim)) {
-                *abort_flag = 1;
-                report_error(p.err, kErrGemmMmaTimeout);
-            }
+            bool ok = mbar_wait_warp(bfull, 0, lim) || fail(kErrGemmMmaTimeout);
             tc_fence_after();
-            for (int t = 0; t < ntiles && !*abort_flag; ++t) {
-                if (!mbar_wait_bounded(&tempty[acc], acc_phase ^ 1, lim)) {
-                    *abort_flag = 1;
-                    report_error(p.err, kErrGemmMmaTimeout);
+            for (int t = 0; ok && t < ntiles && !warp_any(*abort_flag != 0); ++t) {
+                if (!mbar_wait_warp(&tempty[acc], acc_phase ^ 1, lim)) {
+                    ok = fail(kErrGemmMmaTimeout);
                     break;
                 }
                 tc_fence_after();
                 const uint32_t d = tmem_base + static_cast<uint32_t>(acc * kSBN);
                 for (int kb = 0; kb < kblocks; ++kb) {
-                    if (!mbar_wait_bounded(&full[stage], phase, lim)) {
-                        *abort_flag = 1;
-                        report_error(p.err, kErrGemmMmaTimeout);
+                    if (!mbar_wait_warp(&full[stage], phase, lim)) {
+                        ok = fail(kErrGemmMmaTimeout);
                         break;
                     }
                     tc_fence_after();
-                    const uint64_t adesc =
-                        make_sw128_kmajor_desc(smem_u32(smem + C::kAOffset + stage * kSABytes));
-                    const uint64_t bdesc =
-                        make_sw128_kmajor_desc(smem_u32(smem + C::kBOffset + kb * kSBN * 128));
+                    if (elect_one()) {
+                        const uint64_t adesc = make_sw128_kmajor_desc(smem_addr + C::kAOffset + stage * kSABytes);
+                        const uint64_t bdesc = make_sw128_kmajor_desc(smem_addr + C::kBOffset + kb * kSBN * 128);
 #pragma unroll
-                    for (int k = 0; k < kSBK / 16; ++k) {
-                        tc_mma_f16(d, adesc + 2 * k, bdesc + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
+                        for (int k = 0; k < kSBK / 16; ++k) {
+                            tc_mma_f16(d, adesc + 2 * k, bdesc + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
+                        }
+                        tc_commit(&empty[stage]);
+                        if (kb == kblocks - 1) {
+                            tc_commit(&tfull[acc]);
+                        }
                     }
+                    __syncwarp();
                     issued_any = true;
-                    tc_commit(&empty[stage]);
                     if (++stage == kStages) {
                         stage = 0;
                         phase ^= 1;
                     }
                 }
-                if (*abort_flag) {
-                    break;
-                }
-                tc_commit(&tfull[acc]);
                 acc ^= 1;
                 if (acc == 0) {
                     acc_phase ^= 1;
                 }
             }
-            if (*abort_flag && issued_any) {
-                tc_commit(drain);
-                mbar_wait_bounded(drain, 0, kSWaitLimit / 16);
+            if (warp_any(*abort_flag != 0) && issued_any) {
+                if (elect_one()) {
+                    tc_commit(drain);
+                }
+                __syncwarp();
+                mbar_wait_warp(drain, 0, kSWaitLimit / 16);
             }
         }
     } else {
