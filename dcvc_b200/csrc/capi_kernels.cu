@@ -1,6 +1,7 @@
 // extern "C" kernel-level entry points (declared in include/dcvc_b200.h).
 #include "errors.h"
 #include "elementwise.cuh"
+#include "dcb_sm100.cuh"
 #include "ffn_sm100.cuh"
 #include "gemm_sm100.cuh"
 #include "quant_tables.h"
@@ -235,24 +236,40 @@ int dcvc_conv_ffn(int M, int C, int cffn, const void* x, int ldx, const void* w1
                   const void* w2, const float* b2, const void* qscale, void* out, int ldo,
                   int block_n, void* stream)
 {
-    FfnParams p{};
-    p.M = M;
-    p.C = C;
-    p.cffn = cffn;
-    p.b1 = b1;
-    p.b2 = b2;
-    p.qscale = qscale;
-    p.out = out;
-    p.ldo = ldo;
-    p.err = device_error_word();
-    p.block_n = block_n;
-    cudaError_t e = ffn_sm100(x, ldx, w1, w2, p, static_cast<cudaStream_t>(stream));
+    const cudaStream_t st = static_cast<cudaStream_t>(stream);
+    cudaError_t e;
+    if (block_n == 0 && M > 0 && dcb_tail_preferred(M, C, 0, cffn, 4 * cffn)) {
+        const DcbTailParams p{M,  C,  0, cffn, nullptr, 0, x,   ldx, nullptr, w1, w2, nullptr,
+                              b1, b2, qscale, 0, out, ldo, device_error_word()};
+        e = dcb_tail_sm100(DCVC_F16, p, st);
+    } else {
+        const FfnParams p{M, C, cffn, b1, b2, qscale, out, ldo, device_error_word(), block_n};
+        e = ffn_sm100(x, ldx, w1, w2, p, st);
+    }
     if (e == cudaErrorInvalidValue) {
         set_last_error("dcvc_conv_ffn: C must be a multiple of 256 and cffn 128 or 256, block_n "
                        "0, 128 or 256, pitches multiples of 8 elements, pointers 16-byte aligned");
         return kInvalidArgument;
     }
     return cuda_status(e, "dcvc_conv_ffn");
+}
+
+int dcvc_dcb_tail(int dtype, int M, int C, int cdc, int cffn, const void* a, int lda, const void* x, int ldx,
+                  const void* w0, const float* b0, const void* w1, const float* b1, const void* w2,
+                  const float* b2, const void* qscale, int q_rows, void* out, int ldo, void* stream)
+{
+    const DcbTailParams p{M,  C,  cdc, cffn, a,      lda,    x,   ldx, w0, w1, w2, b0,
+                          b1, b2, qscale, q_rows, out, ldo, device_error_word()};
+    cudaError_t e = cudaErrorInvalidValue;
+    if (M > 0 && cdc >= 0 && q_rows >= 0) {
+        e = dcb_tail_sm100(dtype, p, static_cast<cudaStream_t>(stream));
+    }
+    if (e == cudaErrorInvalidValue) {
+        set_last_error("dcvc_dcb_tail: (C, cffn) must be (512, 256), (256, 256) or (256, 128) with cdc 0 or "
+                       "cffn, pitches multiples of 8 elements, pointers 16-byte aligned");
+        return kInvalidArgument;
+    }
+    return cuda_status(e, "dcvc_dcb_tail");
 }
 
 int dcvc_dwconv3x3(const void* x, int H, int W, int C, int ldx, const float* w, void* out, int ldo,

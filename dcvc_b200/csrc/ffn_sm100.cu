@@ -519,15 +519,6 @@ bool ffn_sm100_supported(int C, int cffn, int n1)
     return C > 0 && C % 256 == 0 && (cffn == 128 || cffn == 256) && n1 == 4 * cffn;
 }
 
-bool ffn_sm100_preferred(int C, int cffn, int n1)
-{
-    // With cffn = 256 the fused kernel is slower than the two GEMMs (88 us against 33 + 22 us for
-    // a 512-channel block at 1080p): two 64 KB q buffers leave two 32 KB operand stages, and the
-    // pipeline starves.  With cffn = 128 it is faster (a 256-channel block at 1080p: 22.5 us; the
-    // LD codec gains 8-10 % per frame).
-    return ffn_sm100_supported(C, cffn, n1) && cffn == 128;
-}
-
 cudaError_t ffn_sm100(const void* x, int ldx, const void* w1, const void* w2, const FfnParams& p,
                       cudaStream_t stream)
 {

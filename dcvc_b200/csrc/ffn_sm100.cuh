@@ -21,10 +21,8 @@ struct FfnParams {
     int block_n;         // accumulator columns per item, 128 or 256 (0: the library's choice)
 };
 
-// Whether ffn_sm100 handles a block with these channel counts (n1 = ffn.0 output channels), and
-// whether it is faster there than the two separate GEMMs (the codecs use it only then).
+// Whether ffn_sm100 handles a block with these channel counts (n1 = ffn.0 output channels).
 bool ffn_sm100_supported(int C, int cffn, int n1);
-bool ffn_sm100_preferred(int C, int cffn, int n1);
 
 // out = (quad(x . W1^T + b1) . W2^T + b2 + x) [* qscale] for x [M, C] FP16 (pitch ldx), W1 [4 cffn,
 // C], W2 [C, cffn] dense FP16.  cudaErrorInvalidValue for unsupported shapes or alignments.

@@ -4,8 +4,8 @@
 
 #include <cmath>
 
+#include "dcb_sm100.cuh"
 #include "elementwise.cuh"
-#include "ffn_sm100.cuh"
 #include "gemm_sm100.cuh"
 
 namespace dcvc {
@@ -400,8 +400,17 @@ void run_dcb(Launch& L, const Dcb& d, const __half* x, int ldx, int H, int W, __
     if (!dw_fused) {
         L.note(launch_dwconv3x3(s.t1, H, W, d.cdc, d.cdc, d.dw, s.t2, d.cdc, L.s, d.dtype, img_h));
     }
-    // the FP8 form: the streaming residual GEMM also writes the E4M3 operand of the quad GEMM
     const bool fp8_quad = d.ffn1_w8 != nullptr && s.t5 != nullptr;
+    if (!dw_fused && !fp8_quad && !d.shortcut && d.dc2.dtype == d.dtype && d.ffn1.dtype == d.dtype &&
+        d.ffn2.dtype == d.dtype && dcb_tail_preferred(M, d.C, d.cdc, d.cffn, d.ffn1.cout)) {
+        // everything behind the depthwise 3x3 in one kernel, the two activations between its GEMMs
+        // kept on chip (dcb_sm100.cu)
+        const DcbTailParams tp{M,        d.C,      d.cdc,    d.cffn, s.t2, d.cdc,  xin, ldin, d.dc2.w, d.ffn1.w, d.ffn2.w,
+                               d.dc2.b,  d.ffn1.b, d.ffn2.b, q,      q_rows, out, ldo,  L.err_word};
+        L.note(dcb_tail_sm100(d.dtype, tp, L.s));
+        return;
+    }
+    // the FP8 form: the streaming residual GEMM also writes the E4M3 operand of the quad GEMM
     const bool out8 = fp8_quad && stream_dc2 && d.C % 16 == 0;
     bool t5_ready = false;
     if (dw_fused || out8) {
@@ -432,14 +441,7 @@ void run_dcb(Launch& L, const Dcb& d, const __half* x, int ldx, int H, int W, __
     } else {
         gemm(L, d.dc2, kEpiBiasRes, s.t2, d.cdc, M, s.t3, d.C, xin, ldin);
     }
-    if (!d.shortcut && d.dtype == 0 && (q == nullptr || q_rows == 0) &&
-        ffn_sm100_preferred(d.C, d.cffn, d.ffn1.cout)) {
-        // the ConvFFN as one kernel, the quad output kept on chip (ffn_sm100.cu)
-        FfnParams fp{M, d.C, d.cffn, d.ffn1.b, d.ffn2.b, q, out, ldo, L.err_word, 0};
-        L.note(ffn_sm100(s.t3, d.C, d.ffn1.w, d.ffn2.w, fp, L.s));
-        return;
-    }
-    if (d.ffn1_w8 != nullptr && s.t5 != nullptr) {
+    if (fp8_quad) {
         // the FP8 form: E4M3 copy of the dc output, quad GEMM on kind::f8f6f4
         if (!t5_ready) {
             L.note(launch_quantize_fp8(s.t3, d.dtype, d.C, 1.0f / kFp8ActScale, s.t5, d.C, M, d.C, L.s));

@@ -115,6 +115,24 @@ def conv_ffn(x, w1, b1, w2, b2, qscale=None, out=None, block_n=0):
     return out
 
 
+def dcb_tail(a, x, w0, b0, w1, b1, w2, b2, qscale=None, q_rows=0, out=None):
+    """The part of a DepthConvBlock behind its depthwise 3x3 in one kernel: y = a . w0^T + b0 + x,
+    (quad(y . w1^T + b1) . w2^T + b2 + y) [* qscale]; a = w0 = b0 = None: y = x.  a [M, cdc],
+    x [M, C], weights of the same 16-bit dtype, biases fp32; q_rows > 0: one row of C factors per
+    image of q_rows rows."""
+    M, C = x.shape
+    assert x.stride(1) == 1 and w1.is_contiguous() and w2.is_contiguous()
+    assert a is None or (a.shape[0] == M and a.stride(1) == 1 and w0.is_contiguous())
+    if out is None:
+        out = torch.empty((M, C), dtype=x.dtype, device=x.device)
+    N.check(N.lib.dcvc_dcb_tail(_DT[x.dtype], M, C, a.shape[1] if a is not None else 0, w2.shape[1], _ptr(a),
+                                a.stride(0) if a is not None else 0, x.data_ptr(), x.stride(0), _ptr(w0),
+                                _ptr(b0), w1.data_ptr(), b1.data_ptr(), w2.data_ptr(), b2.data_ptr(),
+                                _ptr(qscale), q_rows, out.data_ptr(), out.stride(0), _stream()),
+            "dcvc_dcb_tail")
+    return out
+
+
 def dwconv3x3(x, H, W, w, out=None):
     """Depthwise 3x3 (pad 1, no bias) over an [H*W, C] NHWC tensor; w is fp32 [9, C]."""
     C = x.shape[1]

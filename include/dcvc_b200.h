@@ -154,6 +154,18 @@ int dcvc_conv_ffn(int M, int C, int cffn, const void* x, int ldx, const void* w1
                   const void* w2, const float* b2, const void* qscale, void* out, int ldo,
                   int block_n, void* stream);
 
+/* The part of a DepthConvBlock behind its depthwise 3x3 in one kernel (layers_proxy.cpp:71-101):
+ *   y = a . w0^T + b0 + x;  t = quad(y . w1^T + b1);  out = (t . w2^T + b2 + y) [* qscale]
+ * with y and t kept on chip.  a [M, cdc] (pitch lda), x, out [M, C] (pitches ldx, ldo; out may be
+ * x), w0 [C, cdc], w1 [4 cffn, C] (rows 4c+k), w2 [C, cffn] of one dtype (DCVC_F16 or DCVC_BF16),
+ * biases FP32; qscale [C] or NULL, with q_rows > 0 one row of C factors per image of q_rows rows.
+ * cdc = 0 (a, w0, b0 unused): y = x, the ConvFFN alone.  (C, cffn) is (512, 256), (256, 256) or
+ * (256, 128), cdc 0 or cffn.  Bit-identical with the dcvc_conv1x1 calls it stands for
+ * (DCVC_EPI_BIAS_RES, DCVC_EPI_QUAD, DCVC_EPI_BIAS_RES / _RES_Q). */
+int dcvc_dcb_tail(int dtype, int M, int C, int cdc, int cffn, const void* a, int lda, const void* x, int ldx,
+                  const void* w0, const float* b0, const void* w1, const float* b1, const void* w2,
+                  const float* b2, const void* qscale, int q_rows, void* out, int ldo, void* stream);
+
 /* Depthwise 3x3, pad 1, no bias, FP32 accumulation: x, out [H*W, C] FP16 (pitches ldx, ldo),
  * w FP32 [9][C] tap-major.  Replaces d3x3 (src/layers/extensions/inference/cutlass/
  * d3x3_kernel.h:104-166, d3x3.cu). */
