@@ -789,133 +789,123 @@ __global__ void __launch_bounds__(kCompactThreads)
 
 // ------------------------------------------------------------------------------ depthwise
 
-// Tiled depthwise 3x3: one CTA computes a kDwTH x kDwTW pixel tile for 64 channels.  The
-// (kDwTH+2) x (kDwTW+2) halo tile is staged in shared memory by 16-byte asynchronous copies
-// (cp.async, zero-filled outside the image), so all of a thread's loads are in flight at once.
-// Each thread then owns one channel pair of kDwRows adjacent tile rows and slides a
-// (kDwRows + 2) x 3 window of FP32 values along them: per column kDwRows + 2 four-byte shared
-// loads feed all of its rows' outputs.
-constexpr int kDwTH = 8;
-constexpr int kDwTW = 32;
-constexpr int kDwCV = 8;  // channel vectors (of 8 halves) per CTA = 64 channels
-constexpr int kDwRows = 2;  // output rows per thread (1: 15.2 us, 2: 13.8 us, 4: 17.6 us at 1080p)
-constexpr int kDwThreads = 32 * (kDwTH / kDwRows);  // 32 channel pairs x row groups
-static_assert(kDwTH % kDwRows == 0, "row groups tile the CTA rows");
+// Depthwise 3x3.  A warp computes a strip of kDwCols columns x kDwRows rows for 64 channels, a lane one
+// channel pair: it walks down kDwRows + 2 input rows, loads kDwCols + 2 pixels of each (one line of 128
+// bytes per pixel and warp, the next row's in flight while this one is summed), converts each value
+// to FP32 once and adds its three products to each of the three output rows it belongs to.  An output
+// row's nine products are summed in the order ky, kx.  Neighbouring strips share columns through L1.
+//
+// What bounds it is instruction issue as much as memory: 9 packed FMAs, 3 conversions, 1.9 loads and
+// stores per output pair.  Strips that touch no border therefore run without a single predicate, and
+// dense tensors of the usual widths (LD > 0) with every column offset an immediate; with run-time
+// strides and per-access bounds checks the same loop issues 68 instructions per output pair instead
+// of 24 and takes 16 us at 1080p.  Against the shared-memory tile kernel this replaces (us, 256
+// channels, old / new): 240 x 136 from L2 12.7 / 6.2, from HBM 13.1 / 9.1, 480 x 270 36.9 / 27.4;
+// other strips at 240 x 136 from HBM: 4 columns x 8 rows 10.9, 4 x 4 10.0, 8 x 8 9.4, 8 x 4 9.1.
+constexpr int kDwCols = 8;
+constexpr int kDwRows = 4;
+constexpr int kDwWarps = 4;
 
-__device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src, int src_bytes)
+struct DwStrip {
+    int W;       // image width
+    int lo, hi;  // the image's rows [lo, hi) in the stack: taps outside read zero
+    int h0, w0;  // the strip's first output row and column
+    int ch;      // this lane's channel pair
+    int ldx, ldo;
+};
+
+// LD: both row pitches when known at compile time, else 0.  EDGE: the strip touches a border.
+template <int DT, int LD, bool EDGE>
+__device__ __forceinline__ void dw_strip(const __half* __restrict__ x, __half* __restrict__ out, const DwStrip& t,
+                                         const float2 (&wp)[9])
 {
-    const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(smem_dst));
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(gmem_src),
-                 "r"(src_bytes)
-                 : "memory");
+    const long long ldx = LD > 0 ? LD : t.ldx, ldo = LD > 0 ? LD : t.ldo;
+    const __half* xr = x + (static_cast<long long>(t.h0 - 1) * t.W + t.w0 - 1) * ldx + t.ch;
+    __half* op = out + (static_cast<long long>(t.h0) * t.W + t.w0) * ldo + t.ch;
+    uint32_t raw[kDwCols + 2];
+    auto load_row = [&](int i) {
+        const bool row = !EDGE || (t.h0 - 1 + i >= t.lo && t.h0 - 1 + i < t.hi);
+#pragma unroll
+        for (int j = 0; j < kDwCols + 2; ++j) {
+            raw[j] = 0;
+            if (!EDGE || (row && static_cast<unsigned>(t.w0 - 1 + j) < static_cast<unsigned>(t.W))) {
+                raw[j] = __ldg(reinterpret_cast<const uint32_t*>(xr + j * ldx));
+            }
+        }
+        xr += t.W * ldx;
+    };
+    load_row(0);
+    float2 acc[3][kDwCols];  // output row r in acc[r % 3]
+#pragma unroll
+    for (int i = 0; i < kDwRows + 2; ++i) {  // input row h0 - 1 + i
+        float2 v[kDwCols + 2];
+#pragma unroll
+        for (int j = 0; j < kDwCols + 2; ++j) {
+            v[j] = Act<DT>::to2(raw[j]);
+        }
+        if (i + 1 < kDwRows + 2) {
+            load_row(i + 1);
+        }
+#pragma unroll
+        for (int j = 0; j < kDwCols; ++j) {
+            float2& up = acc[(i + 1) % 3][j];   // output row i - 2: this is its row below
+            float2& mid = acc[(i + 2) % 3][j];  // output row i - 1
+            float2& dn = acc[i % 3][j];         // output row i: this is its row above
+#pragma unroll
+            for (int kx = 0; kx < 3; ++kx) {
+                if (i >= 2) {
+                    up = __ffma2_rn(v[j + kx], wp[6 + kx], up);
+                }
+                if (i >= 1 && i <= kDwRows) {
+                    mid = __ffma2_rn(v[j + kx], wp[3 + kx], mid);
+                }
+                if (i < kDwRows) {
+                    dn = __ffma2_rn(v[j + kx], wp[kx], kx == 0 ? make_float2(0.f, 0.f) : dn);
+                }
+            }
+            if (i >= 2 && (!EDGE || (t.h0 + i - 2 < t.hi && t.w0 + j < t.W))) {
+                *reinterpret_cast<uint32_t*>(op + j * ldo) = Act<DT>::from2(up.x, up.y);
+            }
+        }
+        if (i >= 2) {
+            op += t.W * ldo;
+        }
+    }
 }
 
-// CUT: the H rows hold images of img_h rows stacked on top of each other; a tap that reaches
-// into the image above or below reads zero, as the padding of each image alone would.
-template <int DT, bool CUT>
-__global__ void __launch_bounds__(kDwThreads) dwconv3x3_kernel(const __half* __restrict__ x, int H,
-                                                               int W, int C, int ldx,
-                                                               const float* __restrict__ wt,
-                                                               __half* __restrict__ out, int ldo,
-                                                               int img_h)
+// grid (strips of all row blocks / kDwWarps, channels / 64).  The H rows hold images of img_h rows
+// stacked on each other; row blocks do not cross images.
+template <int DT, int LD>
+__global__ void __launch_bounds__(32 * kDwWarps, 4)
+    dwconv3x3_kernel(const __half* __restrict__ x, int W, int C, int ldx, const float* __restrict__ wt,
+                     __half* __restrict__ out, int ldo, int img_h, int blocks_per_img, int strips, int total)
 {
     griddep_launch_dependents();
     griddep_wait();
-    __shared__ Vec8h tile[kDwTH + 2][kDwTW + 2][kDwCV];
-    const int c0 = blockIdx.x * kDwCV;  // first channel vector
-    const int h0 = blockIdx.y * kDwTH;
-    const int w0 = blockIdx.z * kDwTW;
-    const int cvecs = C / 8;
-    const int nv = min(kDwCV, cvecs - c0);
-    constexpr int kLoads = (kDwTH + 2) * (kDwTW + 2) * kDwCV;
-#pragma unroll 4
-    for (int i = threadIdx.x; i < kLoads; i += kDwThreads) {
-        const int v = i % kDwCV;
-        const int pix = i / kDwCV;
-        const int tx = pix % (kDwTW + 2);
-        const int ty = pix / (kDwTW + 2);
-        const int h = h0 + ty - 1, w = w0 + tx - 1;
-        const bool in = v < nv && h >= 0 && h < H && w >= 0 && w < W;
-        // out-of-image elements read 0 bytes from a valid address and are zero-filled
-        const __half* src = in ? x + (static_cast<long long>(h) * W + w) * ldx + (c0 + v) * 8 : x;
-        cp_async16(&tile[ty][tx][v], src, in ? 16 : 0);
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    const int cp = threadIdx.x & 31;              // channel pair within the CTA's 64 channels
-    const int ty = kDwRows * (threadIdx.x >> 5);  // first of the thread's tile rows
-    const int ch = c0 * 8 + 2 * cp;         // first of the pair's two channels
-    const bool live = 2 * cp < nv * 8;
-    float2 wp[9];  // the pair's two weights per tap
-    if (live) {
-#pragma unroll
-        for (int k = 0; k < 9; ++k) {
-            wp[k] = __ldg(reinterpret_cast<const float2*>(wt + k * C + ch));
-        }
-    }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();
-    const int ha = h0 + ty;  // the thread's output rows: ha .. ha + kDwRows - 1
-    if (!live || ha >= H) {
+    const int id = blockIdx.x * kDwWarps + (threadIdx.x >> 5);
+    DwStrip t;
+    t.ch = blockIdx.y * 64 + 2 * (threadIdx.x & 31);
+    if (id >= total || t.ch >= C) {
         return;
     }
-    const uint32_t* t2 = reinterpret_cast<const uint32_t*>(&tile[0][0][0]);
-    auto at = [&](int r, int c) { return Act<DT>::to2(t2[(r * (kDwTW + 2) + c) * (4 * kDwCV) + cp]); };
-    bool cut_up[kDwRows], cut_dn[kDwRows];  // the row above / below output row o is another image's
+    const int block = id / strips;
+    const int img = block / blocks_per_img;
+    t.W = W;
+    t.lo = img * img_h;
+    t.hi = t.lo + img_h;
+    t.h0 = t.lo + (block - img * blocks_per_img) * kDwRows;
+    t.w0 = (id - block * strips) * kDwCols;
+    t.ldx = ldx;
+    t.ldo = ldo;
+    float2 wp[9];  // the pair's two weights per tap
 #pragma unroll
-    for (int o = 0; o < kDwRows; ++o) {
-        cut_up[o] = CUT && (ha + o) % img_h == 0;
-        cut_dn[o] = CUT && (ha + o + 1) % img_h == 0;
+    for (int k = 0; k < 9; ++k) {
+        wp[k] = __ldg(reinterpret_cast<const float2*>(wt + k * C + t.ch));
     }
-    float2 win[kDwRows + 2][3];  // window rows ty .. ty + kDwRows + 1 (image rows ha - 1 ..)
-#pragma unroll
-    for (int r = 0; r < kDwRows + 2; ++r) {
-        win[r][0] = at(ty + r, 0);
-        win[r][1] = at(ty + r, 1);
-    }
-    __half* orow = out + static_cast<long long>(ha) * W * ldo + ch;
-    const long long next_row = static_cast<long long>(W) * ldo;
-#pragma unroll
-    for (int tx = 0; tx < kDwTW; ++tx) {
-#pragma unroll
-        for (int r = 0; r < kDwRows + 2; ++r) {
-            win[r][2] = at(ty + r, tx + 2);
-        }
-        // FP32 accumulation in the order ky, kx (d3x3_kernel.h:104-166); one packed FP32 FMA per
-        // tap for the channel pair (each lane rounds as a scalar fmaf would)
-        float2 acc[kDwRows];
-#pragma unroll
-        for (int o = 0; o < kDwRows; ++o) {
-            acc[o] = make_float2(0.f, 0.f);
-        }
-#pragma unroll
-        for (int ky = 0; ky < 3; ++ky) {
-#pragma unroll
-            for (int kx = 0; kx < 3; ++kx) {
-#pragma unroll
-                for (int o = 0; o < kDwRows; ++o) {
-                    float2 v = win[ky + o][kx];
-                    if (CUT && ((ky == 0 && cut_up[o]) || (ky == 2 && cut_dn[o]))) {
-                        v = make_float2(0.f, 0.f);
-                    }
-                    acc[o] = __ffma2_rn(v, wp[ky * 3 + kx], acc[o]);
-                }
-            }
-        }
-        const int w = w0 + tx;
-        if (w < W) {
-            __half* op = orow + static_cast<long long>(w) * ldo;
-#pragma unroll
-            for (int o = 0; o < kDwRows; ++o) {
-                if (ha + o < H) {
-                    *reinterpret_cast<uint32_t*>(op + o * next_row) = Act<DT>::from2(acc[o].x, acc[o].y);
-                }
-            }
-        }
-#pragma unroll
-        for (int r = 0; r < kDwRows + 2; ++r) {
-            win[r][0] = win[r][1];
-            win[r][1] = win[r][2];
-        }
+    if (t.w0 > 0 && t.w0 + kDwCols < W && t.h0 > t.lo && t.h0 + kDwRows < t.hi) {
+        dw_strip<DT, LD, false>(x, out, t, wp);
+    } else {
+        dw_strip<DT, LD, true>(x, out, t, wp);
     }
 }
 
@@ -1350,20 +1340,26 @@ cudaError_t launch_dwconv3x3(const __half* x, int H, int W, int C, int ldx, cons
         (dtype != 0 && dtype != 1) || H % img_h) {
         return cudaErrorInvalidValue;
     }
-    const dim3 grid((C / 8 + kDwCV - 1) / kDwCV, (H + kDwTH - 1) / kDwTH, (W + kDwTW - 1) / kDwTW);
-    const bool cut = img_h < H;
-    if (dtype == 1) {
-        if (cut) {
-            launch_pdl(dwconv3x3_kernel<1, true>, grid, dim3(kDwThreads), 0, s, x, H, W, C, ldx, w, out, ldo, img_h);
-        } else {
-            launch_pdl(dwconv3x3_kernel<1, false>, grid, dim3(kDwThreads), 0, s, x, H, W, C, ldx, w, out, ldo, img_h);
-        }
-    } else {
-        if (cut) {
-            launch_pdl(dwconv3x3_kernel<0, true>, grid, dim3(kDwThreads), 0, s, x, H, W, C, ldx, w, out, ldo, img_h);
-        } else {
-            launch_pdl(dwconv3x3_kernel<0, false>, grid, dim3(kDwThreads), 0, s, x, H, W, C, ldx, w, out, ldo, img_h);
-        }
+    const int strips = (W + kDwCols - 1) / kDwCols, blocks = (img_h + kDwRows - 1) / kDwRows;
+    const long long total = static_cast<long long>(strips) * blocks * (H / img_h);
+    if (total > 0x7fffffff || (C + 63) / 64 > 65535) {
+        return cudaErrorInvalidValue;
+    }
+    const dim3 grid(static_cast<unsigned>((total + kDwWarps - 1) / kDwWarps), (C + 63) / 64);
+    auto launch = [&](auto kernel) {
+        launch_pdl(kernel, grid, dim3(32 * kDwWarps), 0, s, x, W, C, ldx, w, out, ldo, img_h, blocks, strips,
+                   static_cast<int>(total));
+    };
+    // the widths of the codecs' depthwise layers, dense; any other pitch at run time
+    const int ld = ldx == ldo ? ldx : 0;
+    auto by_type = [&](auto f16, auto bf16) { dtype == 0 ? launch(f16) : launch(bf16); };
+    switch (ld) {
+    case 128: by_type(dwconv3x3_kernel<0, 128>, dwconv3x3_kernel<1, 128>); break;
+    case 256: by_type(dwconv3x3_kernel<0, 256>, dwconv3x3_kernel<1, 256>); break;
+    case 384: by_type(dwconv3x3_kernel<0, 384>, dwconv3x3_kernel<1, 384>); break;
+    case 512: by_type(dwconv3x3_kernel<0, 512>, dwconv3x3_kernel<1, 512>); break;
+    case 768: by_type(dwconv3x3_kernel<0, 768>, dwconv3x3_kernel<1, 768>); break;
+    default: by_type(dwconv3x3_kernel<0, 0>, dwconv3x3_kernel<1, 0>); break;
     }
     return cudaGetLastError();
 }
