@@ -60,6 +60,14 @@ __device__ __forceinline__ uint4 lds128(uint32_t addr)
     return v;
 }
 
+// The same for data that nothing writes while `addr` is known: free to move and to be issued early.
+__device__ __forceinline__ float4 lds128_const(uint32_t addr)
+{
+    float4 v;
+    asm("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
+    return v;
+}
+
 __device__ __forceinline__ void sts128(uint32_t addr, uint4 v)
 {
     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
@@ -377,15 +385,33 @@ __device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr)
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 
-// `n` arrivals at once, on this CTA's barrier or on another CTA's.
-__device__ __forceinline__ void mbar_arrive_n(uint64_t* bar, uint32_t n)
+// Predicated forms: a branch around one lane's instruction costs its warp some hundred clocks.
+__device__ __forceinline__ void mbar_arrive_if(bool pred, uint64_t* bar)
 {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(n) : "memory");
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %1, 0;\n\t@p mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}" ::"r"(
+                     smem_u32(bar)),
+                 "r"(static_cast<int>(pred))
+                 : "memory");
 }
 
-__device__ __forceinline__ void mbar_arrive_remote_n(uint32_t cluster_addr, uint32_t n)
+// `n` arrivals at once on a barrier of any CTA of the cluster (address from cluster_map).
+__device__ __forceinline__ void mbar_arrive_remote_if(bool pred, uint32_t cluster_addr, uint32_t n)
 {
-    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0], %1;" ::"r"(cluster_addr), "r"(n) : "memory");
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p mbarrier.arrive.shared::cluster.b64 _, [%0], %1;\n\t}" ::"r"(
+            cluster_addr),
+        "r"(n), "r"(static_cast<int>(pred))
+        : "memory");
+}
+
+__device__ __forceinline__ void tma_store_2d_if(bool pred, const void* tmap, uint32_t src, int c0, int c1)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "@p cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];\n\t}" ::"l"(
+            reinterpret_cast<uint64_t>(tmap)),
+        "r"(src), "r"(c0), "r"(c1), "r"(static_cast<int>(pred))
+        : "memory");
 }
 
 // 2D tiled load into this CTA's shared memory whose completion is counted on a barrier of the

@@ -27,6 +27,7 @@
 
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 
 namespace dcvc {
 
@@ -483,15 +484,9 @@ __global__ void __launch_bounds__(kThreads, 1)
         const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
         int acc = 0;
         uint32_t acc_phase = 0;
-        auto arrive_even = [&](uint64_t* bar, uint32_t n) {  // after a __syncwarp; the even CTA's barrier
-            if (lane == 0) {
-                if (rank == 0) {
-                    mbar_arrive_n(bar, n);
-                } else {
-                    mbar_arrive_remote_n(cluster_map(bar, 0), n);
-                }
-            }
-        };
+        // `n` arrivals on a barrier of the even CTA, after a __syncwarp
+        const uint32_t even = cluster_map(smem, 0) - smem_u32(smem);
+        auto arrive_even = [&](uint64_t* bar, uint32_t n) { mbar_arrive_remote_if(lane == 0, smem_u32(bar) + even, n); };
         auto advance = [&] {
             if (++acc == kAccs) {
                 acc = 0;
@@ -506,7 +501,9 @@ __global__ void __launch_bounds__(kThreads, 1)
             bias[i] = i < G::kB1 ? p.b0[i] : i < G::kB2 ? p.b1[i - G::kB1] : p.b2[i - G::kB2];
         }
         asm volatile("bar.sync 1, %0;" ::"n"(32 * kEpiWarps) : "memory");
-        const uint32_t smem_base = smem_u32(smem), bias_addr = smem_u32(bias);
+        const uint32_t smem_base = smem_u32(smem);
+        uint32_t bias_addr;  // known from here on: reads of the biases cannot move above the barrier
+        asm volatile("mov.u32 %0, %1;" : "=r"(bias_addr) : "r"(smem_u32(bias)) : "memory");
         auto wait_acc = [&] {
             if (!mbar_wait_warp(&accfull[acc], acc_phase, kWaitLimit)) {
                 return fail(kErrGemmEpilogueTimeout);
@@ -521,50 +518,57 @@ __global__ void __launch_bounds__(kThreads, 1)
             arrive_even(&accempty[acc], n);
             advance();
         };
-        // 32 columns of the accumulator plus bias as 16 column pairs
-        auto take = [&](float2 (&v)[16], int col, int b) {
-            uint32_t r[32];
+        auto load_acc = [&](uint32_t (&r)[32], int col) {
             tmem_ld_32x32b_x32(lane_base + kAccCol + acc * kNB + col, r);
-            tc_wait_ld();
+        };
+        // columns 8 j .. 8 j + 7 of loaded accumulators plus bias b
+        auto add_bias = [&](float2 (&v)[4], const uint32_t (&r)[32], int j, int b) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const uint4 bj = lds128(bias_addr + (b + 4 * j) * 4);
-                v[2 * j] = __fadd2_rn(make_float2(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1])),
-                                      make_float2(__uint_as_float(bj.x), __uint_as_float(bj.y)));
-                v[2 * j + 1] = __fadd2_rn(make_float2(__uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3])),
-                                          make_float2(__uint_as_float(bj.z), __uint_as_float(bj.w)));
+            for (int h = 0; h < 2; ++h) {
+                const float4 bj = lds128_const(bias_addr + (b + 8 * j + 4 * h) * 4);
+                const int i = 8 * j + 4 * h;
+                v[2 * h] = __fadd2_rn(make_float2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])),
+                                      make_float2(bj.x, bj.y));
+                v[2 * h + 1] = __fadd2_rn(make_float2(__uint_as_float(r[i + 2]), __uint_as_float(r[i + 3])),
+                                          make_float2(bj.z, bj.w));
             }
         };
         // The residual epilogue of this warp's slab of a block: acc + bias + the slab's row [* q], over
-        // that row.  q: this lane's factors of the slab's columns or null.
-        auto residual_slab = [&](int s, int b, const T* q) {
+        // that row.  q: this lane's factors of the slab's columns (has_q: std::true_type; a run-time
+        // test per value group costs as much as the rest of the group).
+        auto residual_slab = [&](int s, int b, auto has_q, const T* q) {
             const uint32_t line = smem_base + s * kSlabBytes + row * 128;
 #pragma unroll 1
             for (int c = 0; c < 2; ++c) {
-                float2 v[16];
-                take(v, side * 64 + c * 32, b + c * 32);
+                uint32_t r[32];
+                uint4 u[4];
+                load_acc(r, side * 64 + c * 32);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    u[j] = lds128(line + (((c * 4 + j) ^ (row & 7)) << 4));
+                }
+                tc_wait_ld();
                 if (c == 1) {
                     release_acc(2);
                 }
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    const uint32_t cell = line + (((c * 4 + j) ^ (row & 7)) << 4);
-                    const uint4 u = lds128(cell);
-                    v[4 * j + 0] = __fadd2_rn(v[4 * j + 0], P::unpack(u.x));
-                    v[4 * j + 1] = __fadd2_rn(v[4 * j + 1], P::unpack(u.y));
-                    v[4 * j + 2] = __fadd2_rn(v[4 * j + 2], P::unpack(u.z));
-                    v[4 * j + 3] = __fadd2_rn(v[4 * j + 3], P::unpack(u.w));
-                    if (q != nullptr) {
+                    float2 v[4];
+                    add_bias(v, r, j, b + c * 32);
+                    v[0] = __fadd2_rn(v[0], P::unpack(u[j].x));
+                    v[1] = __fadd2_rn(v[1], P::unpack(u[j].y));
+                    v[2] = __fadd2_rn(v[2], P::unpack(u[j].z));
+                    v[3] = __fadd2_rn(v[3], P::unpack(u[j].w));
+                    if constexpr (decltype(has_q)::value) {
                         const uint4 f = __ldg(reinterpret_cast<const uint4*>(q + c * 32 + j * 8));
-                        v[4 * j + 0] = __fmul2_rn(v[4 * j + 0], P::unpack(f.x));
-                        v[4 * j + 1] = __fmul2_rn(v[4 * j + 1], P::unpack(f.y));
-                        v[4 * j + 2] = __fmul2_rn(v[4 * j + 2], P::unpack(f.z));
-                        v[4 * j + 3] = __fmul2_rn(v[4 * j + 3], P::unpack(f.w));
+                        v[0] = __fmul2_rn(v[0], P::unpack(f.x));
+                        v[1] = __fmul2_rn(v[1], P::unpack(f.y));
+                        v[2] = __fmul2_rn(v[2], P::unpack(f.z));
+                        v[3] = __fmul2_rn(v[3], P::unpack(f.w));
                     }
-                    sts128(cell, make_uint4(P::pack(v[4 * j + 0].x, v[4 * j + 0].y),
-                                            P::pack(v[4 * j + 1].x, v[4 * j + 1].y),
-                                            P::pack(v[4 * j + 2].x, v[4 * j + 2].y),
-                                            P::pack(v[4 * j + 3].x, v[4 * j + 3].y)));
+                    sts128(line + (((c * 4 + j) ^ (row & 7)) << 4),
+                           make_uint4(P::pack(v[0].x, v[0].y), P::pack(v[1].x, v[1].y), P::pack(v[2].x, v[2].y),
+                                      P::pack(v[3].x, v[3].y)));
                 }
             }
             fence_proxy_async_smem();
@@ -573,10 +577,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         // xfree of the slab this warp stored last, once its store has read the slab
         int stored = -1;
         auto settle = [&] {
-            if (lane == 0 && stored >= 0) {
-                bulk_wait_read0();
-                mbar_arrive(&xfree[stored]);
-            }
+            bulk_wait_read0();  // lane 0 issued the store
+            mbar_arrive_if(lane == 0 && stored >= 0, &xfree[stored >= 0 ? stored : 0]);
             stored = -1;
         };
         bool ok = true;
@@ -600,7 +602,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                     if (!ok) {
                         break;
                     }
-                    residual_slab(s, s * 64, nullptr);
+                    residual_slab(s, s * 64, std::false_type{}, nullptr);
                     arrive_even(&xfull[s], 1);
                 }
             }
@@ -611,14 +613,16 @@ __global__ void __launch_bounds__(kThreads, 1)
                 if (!ok) {
                     break;
                 }
-                float2 v[16];
-                take(v, grp * 32, G::kB1 + nb * kNB + grp * 32);
+                uint32_t r[32];
+                load_acc(r, grp * 32);
+                tc_wait_ld();
                 release_acc(1);
                 uint32_t o[4];
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
-                    const float2 w0 = wsilu2(v[4 * k + 0]), w1 = wsilu2(v[4 * k + 1]);
-                    const float2 w2 = wsilu2(v[4 * k + 2]), w3 = wsilu2(v[4 * k + 3]);
+                    float2 v[4];
+                    add_bias(v, r, k, G::kB1 + nb * kNB + grp * 32);
+                    const float2 w0 = wsilu2(v[0]), w1 = wsilu2(v[1]), w2 = wsilu2(v[2]), w3 = wsilu2(v[3]);
                     o[k] = P::pack(w0.x + w0.y + w1.x + w1.y, w2.x + w2.y + w3.x + w3.y);
                 }
                 tmem_st_32x32b_x4(lane_base + nb * (kNB / 8) + grp * 4, o);
@@ -640,18 +644,17 @@ __global__ void __launch_bounds__(kThreads, 1)
                 if (!ok) {
                     break;
                 }
-                const T* q = nullptr;
                 if (p.qscale != nullptr) {
                     // this lane's row picks its image's factors in a packed batch
                     const int qm = min(row0 + lane, p.M - 1);
-                    q = reinterpret_cast<const T*>(p.qscale) +
-                        (p.q_rows > 0 ? static_cast<size_t>(qm / p.q_rows) * C : 0) + s * 64;
+                    residual_slab(s, G::kB2 + s * 64, std::true_type{},
+                                  reinterpret_cast<const T*>(p.qscale) +
+                                      (p.q_rows > 0 ? static_cast<size_t>(qm / p.q_rows) * C : 0) + s * 64);
+                } else {
+                    residual_slab(s, G::kB2 + s * 64, std::false_type{}, nullptr);
                 }
-                residual_slab(s, G::kB2 + s * 64, q);
-                if (lane == 0 && row0 < p.M) {
-                    tma_store_2d(&tmO, smem + s * kSlabBytes + quad * 4096, s * 64, row0);
-                    bulk_commit();
-                }
+                tma_store_2d_if(lane == 0 && row0 < p.M, &tmO, smem_base + s * kSlabBytes + quad * 4096, s * 64, row0);
+                bulk_commit();
                 stored = s;
             }
             settle();
