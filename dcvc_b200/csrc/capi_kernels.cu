@@ -120,7 +120,9 @@ int dcvc_conv1x1_f8(int epilogue, int M, int N, int K, const void* a, int lda, c
     p.out = out;
     p.ldo = ldo;
     p.err = device_error_word();
-    cudaError_t e = gemm_sm100(kDtypeF8, a, lda, w, p, epilogue, block_n, static_cast<cudaStream_t>(stream));
+    cudaError_t e = block_n == kBlockNResident
+                        ? cudaErrorInvalidValue
+                        : gemm_sm100(kDtypeF8, a, lda, w, p, epilogue, block_n, static_cast<cudaStream_t>(stream));
     if (e == cudaErrorInvalidValue) {
         set_last_error("dcvc_conv1x1_f8: unsupported shape, pitch, alignment or epilogue");
         return kInvalidArgument;
@@ -175,8 +177,9 @@ int dcvc_conv1x1(int dtype, int epilogue, int M, int N, int K, const void* a, in
     p.sub_w = sub_w;
     p.sub_cout = sub_cout;
     p.err = device_error_word();
-    cudaError_t e = gemm_sm100(dtype, a, lda, w, p, epilogue, block_n,
-                               static_cast<cudaStream_t>(stream));
+    cudaError_t e = block_n == kBlockNResident
+                        ? cudaErrorInvalidValue
+                        : gemm_sm100(dtype, a, lda, w, p, epilogue, block_n, static_cast<cudaStream_t>(stream));
     if (e == cudaErrorInvalidValue) {
         set_last_error("dcvc_conv1x1: unsupported shape, pitch, alignment or epilogue");
         return kInvalidArgument;

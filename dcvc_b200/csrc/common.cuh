@@ -74,6 +74,14 @@ __device__ __forceinline__ void sts128(uint32_t addr, uint4 v)
                  : "memory");
 }
 
+// 32 bytes to 32-byte aligned global memory.
+__device__ __forceinline__ void st_global_256(void* p, const uint32_t (&r)[8])
+{
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(r[0]), "r"(r[1]), "r"(r[2]),
+                 "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+                 : "memory");
+}
+
 // ---------------------------------------------------------------- mbarrier (bounded waits)
 
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count)
@@ -464,6 +472,18 @@ __device__ __forceinline__ void tc_mma_f16_pair_ts(uint32_t tmem_d, uint32_t tme
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
         "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+
+// The same for E4M3 operands (see tc_mma_f8).
+__device__ __forceinline__ void tc_mma_f8_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                               uint32_t accumulate)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
 

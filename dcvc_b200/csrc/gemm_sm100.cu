@@ -811,12 +811,20 @@ cudaError_t gemm_sm100(int dtype, const void* A, int lda, const void* W, const G
     if (bn == 0) {
         // a width measured by the autotuner (gemm_tune.cu) for this shape, else the rule
         bn = gemm_tuned_bn(dtype, epi, p.M, p.N, p.K, epi == kEpiSubpel ? p.sub_w : 0);
+        if (epi == kEpiQuad && g_pair_form.load(std::memory_order_relaxed) == 0 && p.out8 == nullptr &&
+            p.dw_weight == nullptr && quad_sm100_preferred(dtype, p.M, p.N, p.K)) {
+            bn = kBlockNResident;  // 256-wide blocks, as any width recorded for this epilogue
+        }
         if (bn == 0) {
             bn = gemm_pick_bn(p.M, p.N, epi, p.sub_cout, p.K);
             if (bn == kBlockNPair && f8) {
                 bn = 256;  // the pair form is built for 16-bit operands
             }
         }
+    }
+    if (bn == kBlockNResident) {
+        return epi == kEpiQuad && p.out8 == nullptr && p.dw_weight == nullptr ? quad_sm100(dtype, A, lda, W, p, stream)
+                                                                              : cudaErrorInvalidValue;
     }
     if (bn == kBlockNStream) {
         return gemm_stream_sm100(dtype, A, lda, W, p, epi, stream);

@@ -35,6 +35,9 @@ constexpr int kBlockNStream = -1;
 // block_n value selecting the CTA-pair form (cta_group::2, 256 x 256 tiles over two SMs, each
 // staging half of the W tile) of the bias, WSiLU and quad epilogues with 16-bit operands.
 constexpr int kBlockNPair = -2;
+// block_n value of the quad epilogue with resident activations (quad_sm100.cu): the library's own
+// choice only.
+constexpr int kBlockNResident = -3;
 
 struct GemmParams {
     int M, N, K;
@@ -99,6 +102,11 @@ void gemm_set_dw_fusion(bool on);
 // Whether the library's own choice gives the quad GEMM the CTA-pair form (default off).
 void gemm_set_pair_form(bool on);
 bool gemm_dw_fusion_enabled();
+// The quad epilogue with resident activations: K <= 512 16-bit values or 1024 bytes of E4M3 (a multiple
+// of 64, or 256), N a multiple of 256.  Bitwise the same outputs as gemm_sm100.
+bool quad_sm100_eligible(int dtype, int M, int N, int K);
+bool quad_sm100_preferred(int dtype, int M, int N, int K);
+cudaError_t quad_sm100(int dtype, const void* A, int lda, const void* W, const GemmParams& p, cudaStream_t stream);
 cudaError_t gemm_stream_sm100(int dtype, const void* A, int lda, const void* W, const GemmParams& p,
                               int epi, cudaStream_t stream);
 
