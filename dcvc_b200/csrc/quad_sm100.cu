@@ -449,22 +449,27 @@ bool quad_sm100_eligible(int dtype, int M, int N, int K)
            static_cast<long long>((M + 2 * kRows - 1) / (2 * kRows)) * (N / kNB) < 0x7fffffff;
 }
 
-// Whether it is the faster form (us back to back, tiled / this; M x N x K):
+// Whether it is the faster form where no narrower tile runs all at once (gemm_pick_bn; us back to back, tiled / this; M x N x K):
 //   16-bit: 390 x 1024 x 512 6.8 / 6.6, 1560 x 2048 x 512 (56 units on 74 pairs) 7.4 / 7.9,
 //   6240 x 1024 x 512 10.7 / 10.6, 8160 x 2048 x 512 18.3 / 16.9, 32640 x 1024 x 512 30.2 / 28.0, 32640 x
 //   1536 x 384 54.5 / 32.5, 129600 x 1024 x 512 138 / 98
 //   E4M3: 390 x 1024 x 512 6.1 / 5.9, 6240 x 1024 x 512 8.9 / 9.4, 14400 x 1024 x 512 15.1 / 13.3, 32640 24.0 /
 //   20.5, 129600 76.9 / 66.0
-// A unit takes a pair as long as a tile takes one SM in the tiled kernel, so it loses where its units
-// fill the pairs once and badly.
+//   and where the last round of units is nearly empty: 6240 x 1536 x 384 (150 units) 9.8 / 11.2, 3600 x 2048
+//   x 512 (120) 10.0 / 10.6
+// A unit takes a pair about as long as a tile takes one SM in the tiled kernel, so rounds are compared.
 bool quad_sm100_preferred(int dtype, int M, int N, int K)
 {
     if (!quad_sm100_eligible(dtype, M, N, K)) {
         return false;
     }
-    const long long units = static_cast<long long>((M + 2 * kRows - 1) / (2 * kRows)) * (N / kNB);
-    const int pairs = num_sms() / 2;
-    return 2 * units <= pairs || units >= (dtype == kDtypeF8 ? 2 : 1) * pairs;
+    const int sms = num_sms(), pairs = sms / 2;
+    const long long blocks = N / kNB;
+    const long long units = (M + 2 * kRows - 1) / (2 * kRows) * blocks, tiles = (M + kRows - 1) / kRows * blocks;
+    if (dtype == kDtypeF8 && 2 * units <= pairs) {
+        return true;
+    }
+    return 10 * units >= (dtype == kDtypeF8 ? 20 : 17) * pairs && (units + pairs - 1) / pairs <= (tiles + sms - 1) / sms;
 }
 
 cudaError_t quad_sm100(int dtype, const void* A, int lda, const void* W, const GemmParams& p, cudaStream_t stream)

@@ -19,7 +19,7 @@ def _same(a, b):
 
 
 @pytest.mark.parametrize("M,Nn,K", [(1, 256, 64), (128, 1024, 512), (129, 1024, 512), (257, 512, 448), (6400, 1024, 512),
-                                    (9500, 2048, 512), (19000, 1536, 384), (25000, 1024, 256), (33000, 256, 128)])
+                                    (9500, 2048, 512), (9601, 1024, 512), (12700, 1024, 448), (19000, 1536, 384), (25000, 1024, 256), (33000, 256, 128)])
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 def test_16_bit(M, Nn, K, dtype):
     g = torch.Generator(device="cuda").manual_seed(M + Nn + K)
