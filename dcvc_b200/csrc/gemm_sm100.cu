@@ -847,6 +847,24 @@ GemmParams gemm_apply_injection(const GemmParams& p)
     return q;
 }
 
+// Whether CTA pairs (256 x 256 tiles, each CTA staging half of the W tile) beat one CTA per 128 x 256 tile
+// where no narrower tile runs all at once.  A K block of a pair stages 32 KB per CTA instead of 48 KB, which pays
+// once the K loop is long enough to wait on its copies: from K = 512 (us back to back, one CTA / pair: WSiLU
+// 32640 x 256 x 512 12.7 / 11.7, 43200 x 256 x 512 17.7 / 16.1, 32640 x 512 x 512 21.7 / 20.1, bias 32640 x
+// 512 x 1024 34.9 / 29.9, 14400 x 768 x 768 21.0 / 18.3, 8160 x 512 x 1024 11.6 / 11.2; the same at K = 256).
+// The larger tile must not need a round more.
+static bool gemm_pair_preferred(int epi, int M, int N, int K)
+{
+    const long long pairs = num_sms() / 2;
+    if ((epi != kEpiBias && epi != kEpiBiasWsilu) || N % 256 != 0 || K < 512 || pairs < 1) {
+        return false;
+    }
+    const long long cols = N / 256;
+    const long long tiles = (static_cast<long long>(M) + kBM - 1) / kBM * cols;
+    const long long ptiles = (static_cast<long long>(M) + 2 * kBM - 1) / (2 * kBM) * cols;
+    return (ptiles + pairs - 1) / pairs <= (tiles + num_sms() - 1) / num_sms();
+}
+
 // Host launcher.  A: [M, K] with row pitch lda (elements); W: [N, K] dense.  dtype 0 = f16,
 // 1 = bf16, 2 = E4M3 operands with BF16 output.  Returns cudaSuccess or an error
 // (shape/alignment problems -> cudaErrorInvalidValue).
@@ -883,6 +901,9 @@ cudaError_t gemm_sm100(int dtype, const void* A, int lda, const void* W, const G
             }
             if (bn == kBlockNPair && f8) {
                 bn = 256;  // the pair form is built for 16-bit operands
+            }
+            if (bn == 256 && !f8 && gemm_pair_preferred(epi, p.M, p.N, p.K)) {
+                bn = kBlockNPair;
             }
             if (f8 && bn == 64 && p.N % 128 == 0) {
                 bn = 128;  // the narrowest width of the E4M3 form
