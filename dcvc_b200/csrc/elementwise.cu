@@ -7,6 +7,7 @@
 
 #include <algorithm>
 #include <mutex>
+#include <type_traits>
 
 namespace dcvc {
 
@@ -789,8 +790,8 @@ __global__ void __launch_bounds__(kCompactThreads)
 
 // ------------------------------------------------------------------------------ depthwise
 
-// Depthwise 3x3.  A warp computes a strip of kDwCols columns x kDwRows rows for 64 channels, a lane one
-// channel pair: it walks down kDwRows + 2 input rows, loads kDwCols + 2 pixels of each (one line of 128
+// Depthwise 3x3.  A warp computes a strip of kDwCols columns x ROWS rows for 64 channels, a lane one
+// channel pair: it walks down ROWS + 2 input rows, loads kDwCols + 2 pixels of each (one line of 128
 // bytes per pixel and warp, the next row's in flight while this one is summed), converts each value
 // to FP32 once and adds its three products to each of the three output rows it belongs to.  An output
 // row's nine products are summed in the order ky, kx.  Neighbouring strips share columns through L1.
@@ -802,9 +803,12 @@ __global__ void __launch_bounds__(kCompactThreads)
 // of 24 and takes 16 us at 1080p.  Against the shared-memory tile kernel this replaces (us, 256
 // channels, old / new): 240 x 136 from L2 12.7 / 6.2, from HBM 13.1 / 9.1, 480 x 270 36.9 / 27.4;
 // other strips at 240 x 136 from HBM: 4 columns x 8 rows 10.9, 4 x 4 10.0, 8 x 8 9.4, 8 x 4 9.1.
+//
+// A small image is bound by the latency of its rows instead (ROWS + 2 in a chain of two loads each):
+// launch_dwconv3x3 gives it strips of two rows, which read a third more.  The strip's place is found
+// before the dependency wait.
 constexpr int kDwCols = 8;
-constexpr int kDwRows = 4;
-constexpr int kDwWarps = 4;
+constexpr int kDwWarpsPerSm = 16;  // resident at once (128 registers a thread)
 
 struct DwStrip {
     int W;       // image width
@@ -815,7 +819,7 @@ struct DwStrip {
 };
 
 // LD: both row pitches when known at compile time, else 0.  EDGE: the strip touches a border.
-template <int DT, int LD, bool EDGE>
+template <int DT, int LD, int ROWS, bool EDGE>
 __device__ __forceinline__ void dw_strip(const __half* __restrict__ x, __half* __restrict__ out, const DwStrip& t,
                                          const float2 (&wp)[9])
 {
@@ -837,13 +841,13 @@ __device__ __forceinline__ void dw_strip(const __half* __restrict__ x, __half* _
     load_row(0);
     float2 acc[3][kDwCols];  // output row r in acc[r % 3]
 #pragma unroll
-    for (int i = 0; i < kDwRows + 2; ++i) {  // input row h0 - 1 + i
+    for (int i = 0; i < ROWS + 2; ++i) {  // input row h0 - 1 + i
         float2 v[kDwCols + 2];
 #pragma unroll
         for (int j = 0; j < kDwCols + 2; ++j) {
             v[j] = Act<DT>::to2(raw[j]);
         }
-        if (i + 1 < kDwRows + 2) {
+        if (i + 1 < ROWS + 2) {
             load_row(i + 1);
         }
 #pragma unroll
@@ -856,10 +860,10 @@ __device__ __forceinline__ void dw_strip(const __half* __restrict__ x, __half* _
                 if (i >= 2) {
                     up = __ffma2_rn(v[j + kx], wp[6 + kx], up);
                 }
-                if (i >= 1 && i <= kDwRows) {
+                if (i >= 1 && i <= ROWS) {
                     mid = __ffma2_rn(v[j + kx], wp[3 + kx], mid);
                 }
-                if (i < kDwRows) {
+                if (i < ROWS) {
                     dn = __ffma2_rn(v[j + kx], wp[kx], kx == 0 ? make_float2(0.f, 0.f) : dn);
                 }
             }
@@ -873,39 +877,40 @@ __device__ __forceinline__ void dw_strip(const __half* __restrict__ x, __half* _
     }
 }
 
-// grid (strips of all row blocks / kDwWarps, channels / 64).  The H rows hold images of img_h rows
+// grid (strips of all row blocks / WARPS, channels / 64).  The H rows hold images of img_h rows
 // stacked on each other; row blocks do not cross images.
-template <int DT, int LD>
-__global__ void __launch_bounds__(32 * kDwWarps, 4)
+template <int DT, int LD, int ROWS, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS, kDwWarpsPerSm / WARPS)
     dwconv3x3_kernel(const __half* __restrict__ x, int W, int C, int ldx, const float* __restrict__ wt,
                      __half* __restrict__ out, int ldo, int img_h, int blocks_per_img, int strips, int total)
 {
-    griddep_launch_dependents();
-    griddep_wait();
-    const int id = blockIdx.x * kDwWarps + (threadIdx.x >> 5);
+    const int id = blockIdx.x * WARPS + (threadIdx.x >> 5);
     DwStrip t;
     t.ch = blockIdx.y * 64 + 2 * (threadIdx.x & 31);
-    if (id >= total || t.ch >= C) {
-        return;
-    }
     const int block = id / strips;
     const int img = block / blocks_per_img;
     t.W = W;
     t.lo = img * img_h;
     t.hi = t.lo + img_h;
-    t.h0 = t.lo + (block - img * blocks_per_img) * kDwRows;
+    t.h0 = t.lo + (block - img * blocks_per_img) * ROWS;
     t.w0 = (id - block * strips) * kDwCols;
     t.ldx = ldx;
     t.ldo = ldo;
+    asm volatile("" : "+r"(t.h0), "+r"(t.w0), "+r"(t.lo), "+r"(t.hi));
+    griddep_launch_dependents();
+    griddep_wait();
+    if (id >= total || t.ch >= C) {
+        return;
+    }
     float2 wp[9];  // the pair's two weights per tap
 #pragma unroll
     for (int k = 0; k < 9; ++k) {
         wp[k] = __ldg(reinterpret_cast<const float2*>(wt + k * C + t.ch));
     }
-    if (t.w0 > 0 && t.w0 + kDwCols < W && t.h0 > t.lo && t.h0 + kDwRows < t.hi) {
-        dw_strip<DT, LD, false>(x, out, t, wp);
+    if (t.w0 > 0 && t.w0 + kDwCols < W && t.h0 > t.lo && t.h0 + ROWS < t.hi) {
+        dw_strip<DT, LD, ROWS, false>(x, out, t, wp);
     } else {
-        dw_strip<DT, LD, true>(x, out, t, wp);
+        dw_strip<DT, LD, ROWS, true>(x, out, t, wp);
     }
 }
 
@@ -1340,26 +1345,47 @@ cudaError_t launch_dwconv3x3(const __half* x, int H, int W, int C, int ldx, cons
         (dtype != 0 && dtype != 1) || H % img_h) {
         return cudaErrorInvalidValue;
     }
-    const int strips = (W + kDwCols - 1) / kDwCols, blocks = (img_h + kDwRows - 1) / kDwRows;
-    const long long total = static_cast<long long>(strips) * blocks * (H / img_h);
-    if (total > 0x7fffffff || (C + 63) / 64 > 65535) {
+    const int strips = (W + kDwCols - 1) / kDwCols;
+    const long long chunks = (C + 63) / 64;
+    auto strips_of = [&](int rows) { return static_cast<long long>(strips) * ((img_h + rows - 1) / rows) * (H / img_h); };
+    if (strips_of(4) > 0x7fffffff || chunks > 65535) {
         return cudaErrorInvalidValue;
     }
-    const dim3 grid(static_cast<unsigned>((total + kDwWarps - 1) / kDwWarps), (C + 63) / 64);
-    auto launch = [&](auto kernel) {
-        launch_pdl(kernel, grid, dim3(32 * kDwWarps), 0, s, x, W, C, ldx, w, out, ldo, img_h, blocks, strips,
-                   static_cast<int>(total));
+    auto run = [&](auto rows_c, auto warps_c) {
+        constexpr int kRows = decltype(rows_c)::value, kWarps = decltype(warps_c)::value;
+        const int total = static_cast<int>(strips_of(kRows));
+        const dim3 grid((total + kWarps - 1) / kWarps, static_cast<unsigned>(chunks));
+        auto launch = [&](auto kernel) {
+            launch_pdl(kernel, grid, dim3(32 * kWarps), 0, s, x, W, C, ldx, w, out, ldo, img_h, (img_h + kRows - 1) / kRows,
+                       strips, total);
+        };
+        // the widths of the codecs' depthwise layers, dense; any other pitch at run time
+        auto by_width = [&](auto dt) {
+            constexpr int kDt = decltype(dt)::value;
+            switch (ldx == ldo ? ldx : 0) {
+            case 128: return launch(dwconv3x3_kernel<kDt, 128, kRows, kWarps>);
+            case 256: return launch(dwconv3x3_kernel<kDt, 256, kRows, kWarps>);
+            case 384: return launch(dwconv3x3_kernel<kDt, 384, kRows, kWarps>);
+            case 512: return launch(dwconv3x3_kernel<kDt, 512, kRows, kWarps>);
+            case 768: return launch(dwconv3x3_kernel<kDt, 768, kRows, kWarps>);
+            default: return launch(dwconv3x3_kernel<kDt, 0, kRows, kWarps>);
+            }
+        };
+        dtype == 0 ? by_width(std::integral_constant<int, 0>{}) : by_width(std::integral_constant<int, 1>{});
     };
-    // the widths of the codecs' depthwise layers, dense; any other pitch at run time
-    const int ld = ldx == ldo ? ldx : 0;
-    auto by_type = [&](auto f16, auto bf16) { dtype == 0 ? launch(f16) : launch(bf16); };
-    switch (ld) {
-    case 128: by_type(dwconv3x3_kernel<0, 128>, dwconv3x3_kernel<1, 128>); break;
-    case 256: by_type(dwconv3x3_kernel<0, 256>, dwconv3x3_kernel<1, 256>); break;
-    case 384: by_type(dwconv3x3_kernel<0, 384>, dwconv3x3_kernel<1, 384>); break;
-    case 512: by_type(dwconv3x3_kernel<0, 512>, dwconv3x3_kernel<1, 512>); break;
-    case 768: by_type(dwconv3x3_kernel<0, 768>, dwconv3x3_kernel<1, 768>); break;
-    default: by_type(dwconv3x3_kernel<0, 0>, dwconv3x3_kernel<1, 0>); break;
+    // Two-row strips as long as they are all resident at once, in blocks of four warps while there is an
+    // SM for each and of eight from there on (us back to back with four rows and four warps / two rows and
+    // four warps / two rows and eight: 16 x 16 x 512 2.08 / 1.57 / 1.89, 32 x 32 x 384 2.34 / 1.96 /
+    // 2.29, 30 x 52 x 256 2.42 / 2.03 / 2.44, 45 x 80 x 512 3.80 / 3.16 / 2.71, 90 x 160 x 128 3.69 / 3.13
+    // / 2.69; past that 68 x 120 x 512 4.70 / 5.04 / 5.29, 270 x 480 x 256 27.8 / 31.0 / 34.2).
+    const long long warps = strips_of(2) * chunks;
+    using std::integral_constant;
+    if (warps > static_cast<long long>(kDwWarpsPerSm) * num_sms()) {
+        run(integral_constant<int, 4>{}, integral_constant<int, 4>{});
+    } else if ((strips_of(2) + 3) / 4 * chunks <= num_sms()) {
+        run(integral_constant<int, 2>{}, integral_constant<int, 4>{});
+    } else {
+        run(integral_constant<int, 2>{}, integral_constant<int, 8>{});
     }
     return cudaGetLastError();
 }

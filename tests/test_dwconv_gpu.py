@@ -39,3 +39,12 @@ def test_strip_edges(h, w, images, c, pad, dtype):
     bound = (1 + ulp) * 9 * 2.0 ** -24 * mag + ulp * ref.abs() + 2.0 ** -24
     assert bool(((out.double() - ref).abs() <= bound).all())
     assert bool(torch.isnan(buf[:, c:]).all())
+
+
+@pytest.mark.parametrize("h,w,images,c", [(21, 29, 1, 256), (45, 43, 1, 512), (23, 41, 2, 512), (64, 120, 1, 128), (62, 73, 1, 384),
+                                          (101, 131, 1, 768), (67, 119, 2, 256), (98, 120, 1, 264)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_strip_forms(h, w, images, c, dtype):
+    """Sizes on both sides of the points where strips of two rows go from blocks of four warps to eight
+    and then give way to strips of four rows."""
+    test_strip_edges(h, w, images, c, 0, dtype)
