@@ -2,13 +2,15 @@
 
 These exist for tests and for callers that compose their own graphs; the codec runtime itself
 drives the kernels from C++.  Every wrapper runs the sm_100a kernel through libdcvc_b200.so on
-the current CUDA stream; nothing here falls back to PyTorch math.
+the current CUDA stream; nothing here falls back to PyTorch math.  The wrappers of the layers' hot
+operators go through _torch_calls (csrc/python/torch_calls.cpp), the others through ctypes.
 """
 import ctypes
 
 import torch
 
 from . import _native as N
+from . import _torch_calls as _calls  # after torch, whose libraries it needs
 
 _DT = {torch.float16: N.F16, torch.bfloat16: N.BF16}
 
@@ -18,7 +20,17 @@ def _ptr(t):
 
 
 def _stream():
-    return torch.cuda.current_stream().cuda_stream
+    # the handle behind torch.cuda.current_stream(), without a Stream object for each call (3.3 us, 0.3)
+    if not torch.cuda.is_initialized():
+        return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
+def _done(out, where):
+    """The output of a _torch_calls function, or the error for the status it returned instead."""
+    if out.__class__ is int:
+        N.check(out, where)
+    return out
 
 
 def conv1x1(a, w, bias=None, epilogue=N.EPI_BIAS, res=None, res2=None, qscale=None, out=None,
@@ -28,22 +40,8 @@ def conv1x1(a, w, bias=None, epilogue=N.EPI_BIAS, res=None, res2=None, qscale=No
     bias is fp32 [N]; res/res2 are [M, N] views; qscale is [N] in the activation dtype.
     QUAD returns [M, N/4]; SUBPEL returns [4*M, sub_cout] (the 2x pixel-shuffled grid).
     """
-    assert a.dim() == 2 and a.stride(1) == 1 and w.is_contiguous()
-    M, K = a.shape
-    Nn = w.shape[0]
-    if out is None:
-        if epilogue == N.EPI_QUAD:
-            out = torch.empty((M, Nn // 4), dtype=a.dtype, device=a.device)
-        elif epilogue == N.EPI_SUBPEL:
-            out = torch.empty((4 * M, sub_cout), dtype=a.dtype, device=a.device)
-        else:
-            out = torch.empty((M, Nn), dtype=a.dtype, device=a.device)
-    N.check(N.lib.dcvc_conv1x1(
-        _DT[a.dtype], epilogue, M, Nn, K, a.data_ptr(), a.stride(0), w.data_ptr(), _ptr(bias),
-        _ptr(res), res.stride(0) if res is not None else 0,
-        _ptr(res2), res2.stride(0) if res2 is not None else 0, _ptr(qscale),
-        out.data_ptr(), out.stride(0), sub_w, sub_cout, block_n, _stream()), "dcvc_conv1x1")
-    return out
+    return _done(_calls.conv1x1(a, w, bias, epilogue, res, res2, qscale, out, sub_w, sub_cout, block_n),
+                 "dcvc_conv1x1")
 
 
 def quantize_fp8(x, inv_scale, out=None):
@@ -62,16 +60,7 @@ def conv1x1_f8(a, w, wscale, bias, epilogue=N.EPI_BIAS, out=None, block_n=0):
     """The FP8 GEMM form: a [M, K] and w [N, K] float8_e4m3fn, wscale [N] fp32 (activation scale
     times weight-row scale), bias [N] fp32; returns bfloat16 epilogue(acc * wscale + bias)
     ([M, N/4] for the QUAD epilogue)."""
-    assert a.dim() == 2 and a.stride(1) == 1 and w.is_contiguous()
-    M, K = a.shape
-    Nn = w.shape[0]
-    if out is None:
-        out = torch.empty((M, Nn // 4 if epilogue == N.EPI_QUAD else Nn), dtype=torch.bfloat16,
-                          device=a.device)
-    N.check(N.lib.dcvc_conv1x1_f8(epilogue, M, Nn, K, a.data_ptr(), a.stride(0), w.data_ptr(),
-                                  wscale.data_ptr(), bias.data_ptr(), out.data_ptr(), out.stride(0),
-                                  block_n, _stream()), "dcvc_conv1x1_f8")
-    return out
+    return _done(_calls.conv1x1_f8(a, w, wscale, bias, epilogue, out, block_n), "dcvc_conv1x1_f8")
 
 
 def gemm_autotune(dtype, epilogue, M, Nn, K, sub_w=0, sub_cout=0):
@@ -103,16 +92,7 @@ def gemm_tuning_clear():
 def conv_ffn(x, w1, b1, w2, b2, qscale=None, out=None, block_n=0):
     """Fused ConvFFN: (quad(x . w1^T + b1) . w2^T + b2 + x) [* qscale] for x [M, C] fp16;
     w1 [4 cffn, C], w2 [C, cffn] fp16, b1 / b2 fp32."""
-    assert x.dim() == 2 and x.stride(1) == 1 and w1.is_contiguous() and w2.is_contiguous()
-    M, C = x.shape
-    cffn = w2.shape[1]
-    if out is None:
-        out = torch.empty((M, C), dtype=x.dtype, device=x.device)
-    N.check(N.lib.dcvc_conv_ffn(M, C, cffn, x.data_ptr(), x.stride(0), w1.data_ptr(),
-                                b1.data_ptr(), w2.data_ptr(), b2.data_ptr(), _ptr(qscale),
-                                out.data_ptr(), out.stride(0), block_n, _stream()),
-            "dcvc_conv_ffn")
-    return out
+    return _done(_calls.conv_ffn(x, w1, b1, w2, b2, qscale, out, block_n), "dcvc_conv_ffn")
 
 
 def dcb_tail(a, x, w0, b0, w1, b1, w2, b2, qscale=None, q_rows=0, out=None):
@@ -124,7 +104,7 @@ def dcb_tail(a, x, w0, b0, w1, b1, w2, b2, qscale=None, q_rows=0, out=None):
     assert x.stride(1) == 1 and w1.is_contiguous() and w2.is_contiguous()
     assert a is None or (a.shape[0] == M and a.stride(1) == 1 and w0.is_contiguous())
     if out is None:
-        out = torch.empty((M, C), dtype=x.dtype, device=x.device)
+        out = x.new_empty((M, C))
     N.check(N.lib.dcvc_dcb_tail(_DT[x.dtype], M, C, a.shape[1] if a is not None else 0, w2.shape[1], _ptr(a),
                                 a.stride(0) if a is not None else 0, x.data_ptr(), x.stride(0), _ptr(w0),
                                 _ptr(b0), w1.data_ptr(), b1.data_ptr(), w2.data_ptr(), b2.data_ptr(),
@@ -135,22 +115,12 @@ def dcb_tail(a, x, w0, b0, w1, b1, w2, b2, qscale=None, q_rows=0, out=None):
 
 def dwconv3x3(x, H, W, w, out=None):
     """Depthwise 3x3 (pad 1, no bias) over an [H*W, C] NHWC tensor; w is fp32 [9, C]."""
-    C = x.shape[1]
-    if out is None:
-        out = torch.empty_like(x)
-    N.check(N.lib.dcvc_dwconv3x3(x.data_ptr(), H, W, C, x.stride(0), w.data_ptr(), out.data_ptr(),
-                                 out.stride(0), _stream()), "dcvc_dwconv3x3")
-    return out
+    return _done(_calls.dwconv3x3(x, H, W, w, 0, out), "dcvc_dwconv3x3")
 
 
 def dwconv3x3_ex(x, H, W, w, img_h=0, out=None):
     """dwconv3x3 for FP16 or BF16 x over images of img_h rows stacked along H (0: one image)."""
-    C = x.shape[1]
-    if out is None:
-        out = torch.empty_like(x)
-    N.check(N.lib.dcvc_dwconv3x3_ex(_DT[x.dtype], x.data_ptr(), H, W, img_h, C, x.stride(0), w.data_ptr(),
-                                    out.data_ptr(), out.stride(0), _stream()), "dcvc_dwconv3x3_ex")
-    return out
+    return _done(_calls.dwconv3x3_ex(x, H, W, w, img_h, out), "dcvc_dwconv3x3_ex")
 
 
 def dw3x3_conv1x1_res(x, H, W, dw_w, w, bias, res, img_h=0, out=None):
@@ -160,7 +130,7 @@ def dw3x3_conv1x1_res(x, H, W, dw_w, w, bias, res, img_h=0, out=None):
     Nn = w.shape[0]
     assert M == H * W and w.shape[1] == K and w.is_contiguous() and dw_w.is_contiguous()
     if out is None:
-        out = torch.empty((M, Nn), dtype=x.dtype, device=x.device)
+        out = x.new_empty((M, Nn))
     N.check(N.lib.dcvc_dw3x3_conv1x1_res(_DT[x.dtype], H, W, img_h, x.data_ptr(), x.stride(0), dw_w.data_ptr(),
                                          K, w.data_ptr(), Nn, bias.data_ptr(), res.data_ptr(), res.stride(0),
                                          out.data_ptr(), out.stride(0), _stream()), "dcvc_dw3x3_conv1x1_res")
