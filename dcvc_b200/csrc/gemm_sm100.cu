@@ -57,7 +57,7 @@ __host__ __device__ constexpr bool epi_has_q(int e) { return e == kEpiBiasResQ |
 // columns each) otherwise, which leaves shared memory for a deeper operand pipeline.
 __host__ __device__ constexpr int epi_warps(int bn, int epi)
 {
-    return (epi_has_res(epi) && bn >= 128) ? 16 : 8;
+    return bn == 32 ? 4 : (epi_has_res(epi) && bn >= 128) ? 16 : 8;
 }
 // Accumulator columns per epilogue warp, and output columns of one store box (32 rows high).
 __host__ __device__ constexpr int epi_cols(int bn, int epi) { return bn / (epi_warps(bn, epi) / 4); }
@@ -93,10 +93,11 @@ struct GemmCfg {
     static constexpr int kEpiBytes = kEpiWarps * kWarpStage;
     static constexpr int kABytes = kBM * kBK * 2;
     static constexpr int kBBytes = (PAIR ? BN / 2 : BN) * kBK * 2;
-    // K blocks per ring stage: a stage costs its MMA issuer some 400 clocks, two blocks of 128 x 128 x 64
-    // run for 570 and of 128 x 64 x 64 for less (small GEMMs are a chain of stages: K = 768, 390 rows
-    // on 64-wide tiles 5.6 us with one block per stage, 4.6 with two)
-    static constexpr int kStageTiles = BN <= 128 ? 2 : 1;
+    // K blocks per ring stage, at most: a stage costs its MMA issuer some 400 clocks; two blocks of 128 x
+    // 128 x 64 run for 570, four of 128 x 64 x 64 for 1000, and a small GEMM is a chain of stages (390 x 768
+    // x 768 residual on 64-wide tiles 5.6 us with one block per stage, 4.6 with two; 256 x 512 x 1536 on
+    // 32-wide ones 6.4 with two, 5.7 with four).
+    static constexpr int kStageTiles = BN <= 64 ? 4 : BN <= 128 ? 2 : 1;
     static constexpr int kTileBytes = kABytes + kBBytes;
     static constexpr int kStageBytes = kStageTiles * kTileBytes;
     static constexpr int kBarBytes = 512;
@@ -216,6 +217,10 @@ __global__ void __launch_bounds__(GemmCfg<BN, EPI, PAIR>::kThreads, 1)
     // 5.87 -> 5.32, 8160 x 512 x 512 8.77 -> 8.30, 32640 x 512 x 512 WSiLU 19.8 -> 19.4 (back to back).
     int first_m = (unit % num_m) * kTileM + row_off, first_n = (unit / num_m) * BN;
     int kb_end = kblocks;
+    // K blocks per stage: the fewest stages, evenly filled (K = 384: 3 + 3)
+    const int per = C::kStageTiles <= 2 ? C::kStageTiles
+                                        : (kblocks + (kblocks + C::kStageTiles - 1) / C::kStageTiles - 1) /
+                                              ((kblocks + C::kStageTiles - 1) / C::kStageTiles);
     asm volatile("" : "+r"(first_m), "+r"(first_n), "+r"(kb_end));
     // setup above overlaps the predecessor's tail; its outputs are read only after this
     griddep_launch_dependents();
@@ -239,8 +244,8 @@ __global__ void __launch_bounds__(GemmCfg<BN, EPI, PAIR>::kThreads, 1)
             bool ok = true;
             int m0 = first_m, n0 = first_n;
             for (int tile = unit; ok && tile < num_tiles;) {
-                for (int kb = 0; kb < kb_end; kb += C::kStageTiles) {
-                    const int tiles = min(C::kStageTiles, kb_end - kb);
+                for (int kb = 0; kb < kb_end; kb += per) {
+                    const int tiles = min(per, kb_end - kb);
                     // (the first round finds every stage free)
                     if (issued >= kStages && !mbar_wait_warp(&empty[stage], phase ^ 1, lim)) {
                         ok = fail(kErrGemmProducerTimeout);
@@ -317,8 +322,8 @@ __global__ void __launch_bounds__(GemmCfg<BN, EPI, PAIR>::kThreads, 1)
                 }
                 tc_fence_after();
                 const uint32_t d = tmem_base + static_cast<uint32_t>(acc * BN);
-                for (int kb = 0; kb < kblocks; kb += C::kStageTiles) {
-                    const int tiles = min(C::kStageTiles, kblocks - kb);
+                for (int kb = 0; kb < kblocks; kb += per) {
+                    const int tiles = min(per, kblocks - kb);
                     if (!ready && !mbar_wait_warp(&full[stage], phase, lim)) {
                         ok = fail(kErrGemmMmaTimeout);
                         break;
@@ -355,7 +360,7 @@ __global__ void __launch_bounds__(GemmCfg<BN, EPI, PAIR>::kThreads, 1)
                         } else {
                             tc_commit(&empty[stage]);
                         }
-                        if (kb + C::kStageTiles >= kblocks) {
+                        if (kb + per >= kblocks) {
                             if constexpr (PAIR) {
                                 tc_commit_pair_both(&tfull[acc]);
                             } else {
@@ -436,7 +441,7 @@ __global__ void __launch_bounds__(GemmCfg<BN, EPI, PAIR>::kThreads, 1)
         // The bias of the next 32 columns is loaded ahead: a tile's first while its accumulator is being
         // computed, the others during the columns before (500 clocks of L2 latency each otherwise; not
         // where 16 warps leave no registers for it).
-        constexpr bool kBiasAhead = EPI != kEpiSubpel && (C::kEpiWarps == 8 || (EPI == kEpiBiasRes && BN == 128));
+        constexpr bool kBiasAhead = EPI != kEpiSubpel && (C::kEpiWarps <= 8 || (EPI == kEpiBiasRes && BN == 128));
         float4 bb[8];
         auto load_bias = [&](int col) {
             const float4* b4 = reinterpret_cast<const float4*>(p.bias + col);
@@ -508,6 +513,7 @@ __global__ void __launch_bounds__(GemmCfg<BN, EPI, PAIR>::kThreads, 1)
                 }
             } else if constexpr (C::kDirect) {
                 // quad: 32 columns -> 8 outputs of this lane's row at a time
+                static_assert(kBiasAhead, "the bias is in registers by now");
                 const int m = row0 + lane;
 #pragma unroll 1
                 for (int c = 0; c < C::kCols / 32; ++c) {
@@ -822,11 +828,13 @@ int gemm_pick_bn(int M, int N, int epi, int sub_cout, int K)
     // which falls with the width: the narrowest width with at most one tile per SM (us at 256 / 128 /
     // 64 columns: 390 x 768 x 768 residual 8.4 / 6.6 / 5.6, 1024 x 512 x 512 residual 7.3 / 5.6 / 4.7, 1024 x
     // 256 x 512 WSiLU 7.3 / 5.6 / 4.7; one step too narrow costs a second round: 3600 x 512 x 512 residual
-    // 7.8 / 6.0 / 7.1, 6240 x 768 x 768 WSiLU 9.4 / 10.6 / 15.5).  The width changes no output bit.  Quad:
+    // 7.8 / 6.0 / 7.1, 6240 x 768 x 768 WSiLU 9.4 / 10.6 / 15.5; at 64 / 32 columns, with later kernels: 390 x
+    // 768 x 768 residual 4.84 / 4.17, 1024 x 384 x 384 3.80 / 3.34, 256 x 2048 x 512 quad 3.72 / 3.33).  The
+    // width changes no output bit.  32 columns are the library's choice only, where 64 divide N too.  Quad:
     // see also quad_sm100_preferred.
     const long long rows = (M + kBM - 1) / kBM;
-    for (int bn : {64, 128, 256}) {
-        if (fits(bn) && rows * (N / bn) <= num_sms()) {
+    for (int bn : {32, 64, 128, 256}) {
+        if (fits(bn) && (bn > 32 || fits(64)) && rows * (N / bn) <= num_sms()) {
             return bn;
         }
     }
@@ -929,7 +937,7 @@ cudaError_t gemm_sm100(int dtype, const void* A, int lda, const void* W, const G
             if (bn == 256 && !f8 && gemm_pair_preferred(epi, p.M, p.N, p.K)) {
                 bn = kBlockNPair;
             }
-            if (f8 && bn == 64 && p.N % 128 == 0) {
+            if (f8 && (bn == 32 || bn == 64) && p.N % 128 == 0) {
                 bn = 128;  // the narrowest width of the E4M3 form
             }
         }
@@ -952,7 +960,7 @@ cudaError_t gemm_sm100(int dtype, const void* A, int lda, const void* W, const G
         }
         bn = 256;
     }
-    if (bn <= 0 || p.N % bn != 0) {
+    if (bn <= 0 || p.N % bn != 0 || (bn == 32 && !chosen)) {
         return cudaErrorInvalidValue;
     }
     if (epi != kEpiSubpel && p.bias == nullptr) {
@@ -1029,12 +1037,14 @@ cudaError_t gemm_sm100(int dtype, const void* A, int lda, const void* W, const G
         case 256: return dispatch_epi<__half, 256>(epi, m, p, stream);
         case 128: return dispatch_epi<__half, 128>(epi, m, p, stream);
         case 64: return dispatch_epi<__half, 64>(epi, m, p, stream);
+        case 32: return dispatch_epi<__half, 32>(epi, m, p, stream);
         }
     } else {
         switch (bn) {
         case 256: return dispatch_epi<__nv_bfloat16, 256>(epi, m, p, stream);
         case 128: return dispatch_epi<__nv_bfloat16, 128>(epi, m, p, stream);
         case 64: return dispatch_epi<__nv_bfloat16, 64>(epi, m, p, stream);
+        case 32: return dispatch_epi<__nv_bfloat16, 32>(epi, m, p, stream);
         }
     }
     return cudaErrorInvalidValue;
