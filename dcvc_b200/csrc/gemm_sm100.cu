@@ -882,19 +882,23 @@ GemmParams gemm_apply_injection(const GemmParams& p)
 // Whether CTA pairs (256 x 256 tiles, each CTA staging half of the W tile) beat one CTA per 128 x 256 tile
 // where no narrower tile runs all at once.  A K block of a pair stages 32 KB per CTA instead of 48 KB, which pays
 // once the K loop is long enough to wait on its copies: from K = 512 (us back to back, one CTA / pair: WSiLU
-// 32640 x 256 x 512 12.7 / 11.7, 43200 x 256 x 512 17.7 / 16.1, 32640 x 512 x 512 21.7 / 20.1, bias 32640 x
-// 512 x 1024 34.9 / 29.9, 14400 x 768 x 768 21.0 / 18.3, 8160 x 512 x 1024 11.6 / 11.2; the same at K = 256).
-// The larger tile must not need a round more.
+// 14400 x 512 x 512 12.6 / 11.6, 14400 x 768 x 768 20.7 / 18.0, 32640 x 512 x 512 21.2 / 19.2, residual 14400 x
+// 512 x 512 15.7 / 14.4, 32640 x 512 x 512 27.7 / 22.7, 32640 x 768 x 768 56.2 / 44.8; at K = 256 WSiLU 32640 x
+// 256 10.2 / 10.4).  The larger tile must not need a round more (6240 x 768 x 768 10.0 / 12.5), and where one
+// CTA per tile runs in one round only the residual epilogues gain, whose pairs have more stages beside the
+// residual (8160 x 512 x 512 WSiLU 8.7 / 9.0, residual 10.4 / 10.1).
 static bool gemm_pair_preferred(int epi, int M, int N, int K)
 {
     const long long pairs = num_sms() / 2;
-    if ((epi != kEpiBias && epi != kEpiBiasWsilu) || N % 256 != 0 || K < 512 || pairs < 1) {
+    const bool res = epi == kEpiBiasRes || epi == kEpiBiasResQ;
+    if ((epi != kEpiBias && epi != kEpiBiasWsilu && !res) || N % 256 != 0 || K < 512 || pairs < 1) {
         return false;
     }
     const long long cols = N / 256;
     const long long tiles = (static_cast<long long>(M) + kBM - 1) / kBM * cols;
     const long long ptiles = (static_cast<long long>(M) + 2 * kBM - 1) / (2 * kBM) * cols;
-    return (ptiles + pairs - 1) / pairs <= (tiles + num_sms() - 1) / num_sms();
+    const long long rounds = (tiles + num_sms() - 1) / num_sms();
+    return (res || rounds > 1) && (ptiles + pairs - 1) / pairs <= rounds;
 }
 
 // Host launcher.  A: [M, K] with row pitch lda (elements); W: [N, K] dense.  dtype 0 = f16,
@@ -955,7 +959,8 @@ cudaError_t gemm_sm100(int dtype, const void* A, int lda, const void* W, const G
     }
     const bool pair = bn == kBlockNPair;
     if (pair) {
-        if (f8 || (epi != kEpiBias && epi != kEpiBiasWsilu && epi != kEpiQuad) || num_sms() < 2) {
+        const bool res = epi == kEpiBiasRes || epi == kEpiBiasResQ;  // the library's choice only
+        if (f8 || (epi != kEpiBias && epi != kEpiBiasWsilu && epi != kEpiQuad && !(res && chosen)) || num_sms() < 2) {
             return cudaErrorInvalidValue;
         }
         bn = 256;
@@ -1021,6 +1026,12 @@ cudaError_t gemm_sm100(int dtype, const void* A, int lda, const void* W, const G
         case kEpiBiasWsilu:
             return dtype == 0 ? launch_one<__half, 256, kEpiBiasWsilu, false, true>(m, p, stream)
                               : launch_one<__nv_bfloat16, 256, kEpiBiasWsilu, false, true>(m, p, stream);
+        case kEpiBiasRes:
+            return dtype == 0 ? launch_one<__half, 256, kEpiBiasRes, false, true>(m, p, stream)
+                              : launch_one<__nv_bfloat16, 256, kEpiBiasRes, false, true>(m, p, stream);
+        case kEpiBiasResQ:
+            return dtype == 0 ? launch_one<__half, 256, kEpiBiasResQ, false, true>(m, p, stream)
+                              : launch_one<__nv_bfloat16, 256, kEpiBiasResQ, false, true>(m, p, stream);
         case kEpiQuad:
             return dtype == 0 ? launch_one<__half, 256, kEpiQuad, false, true>(m, p, stream)
                               : launch_one<__nv_bfloat16, 256, kEpiQuad, false, true>(m, p, stream);

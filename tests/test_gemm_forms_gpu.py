@@ -65,3 +65,27 @@ def test_narrow_tiles_are_the_librarys_choice():
         ops.conv1x1(a, w, b, block_n=32)
     with pytest.raises(N.DcvcError):
         ops.conv1x1(a, w[:96].contiguous(), b)  # no width for N = 96
+
+
+@pytest.mark.parametrize("M,Nn,K", [(4737, 512, 512), (8160, 512, 512), (8193, 512, 576), (9473, 512, 512), (8160, 768, 768), (19000, 256, 512), (19073, 256, 1024),
+                                    (6240, 768, 768), (9601, 512, 448)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("with_q", [False, True])
+def test_residual_pairs(M, Nn, K, dtype, with_q):
+    """The residual epilogues on CTA pairs, and around the sizes where the library takes them."""
+    g = torch.Generator(device="cuda").manual_seed(M + Nn + K)
+    a = torch.randn(M, K, device="cuda", generator=g).to(dtype)
+    w = (torch.randn(Nn, K, device="cuda", generator=g) * K ** -0.5).to(dtype)
+    b = torch.randn(Nn, device="cuda", generator=g) * 0.3
+    res = torch.randn(M, Nn + 8, device="cuda", generator=g).to(dtype)[:, 8:]
+    q = (torch.rand(Nn, device="cuda", generator=g) + 0.5).to(dtype) if with_q else None
+    epi = N.EPI_BIAS_RES_Q if with_q else N.EPI_BIAS_RES
+    ref = ops.conv1x1(a, w, b, epi, res=res, qscale=q, block_n=128)
+    buf = torch.full((M, Nn + 16), float("nan"), device="cuda", dtype=dtype)
+    out = ops.conv1x1(a, w, b, epi, res=res, qscale=q, out=buf[:, 8:8 + Nn])
+    torch.cuda.synchronize()
+    assert N.device_error() == 0
+    assert torch.equal(out.contiguous().view(torch.int16), ref.view(torch.int16))
+    assert bool(torch.isnan(buf[:, :8]).all()) and bool(torch.isnan(buf[:, 8 + Nn:]).all())
+    with pytest.raises(N.DcvcError):  # callers cannot ask for it
+        ops.conv1x1(a, w, b, epi, res=res, qscale=q, block_n=N.BLOCK_N_PAIR)
