@@ -12,15 +12,15 @@
 // tensor memory (the A operand of ffn.2), and each CTA stages half of every weight tile, so the
 // weights cross L2 once per 256 rows.
 //
-// Per tile the MMA warp of the even CTA walks blocks of output columns - dc.3's, ffn.0's, ffn.2's -
-// each into one of two accumulators while twelve epilogue warps (32 rows x 64 columns, one slab
-// wide) drain the block before.  Blocks are 192 wide (128 at the end): an MMA of this shape reads
-// 4 KB of activations and N / 2 x 32 bytes of weights from each SM's shared memory in N / 2 clocks, and
-// the weight copies write as much again, so 128-wide blocks use up shared memory's 128 bytes a
-// clock (measured 70 clocks an MMA instead of 64, and every epilogue access waiting), 256-wide
-// ones would leave no tensor memory for t.  The FP32 sums run over K in the same order as in the
-// separate GEMMs and each epilogue applies the same operations in the same order, with x and t
-// rounded to 16 bits where the separate launches stored them, so the result is bitwise theirs.
+// Per tile the MMA warp of the even CTA walks blocks of 128 output columns - dc.3's, ffn.0's, ffn.2's -
+// each into one of three accumulators while sixteen epilogue warps drain the blocks before.  An MMA of
+// this shape reads 4 KB of activations and 2 KB of weights from each SM's shared memory in 64 clocks and
+// the weight copies write as much again, so the blocks use up most of shared memory's 128 bytes a
+// clock (measured 70 clocks an MMA); 192-wide blocks in two accumulators leave the epilogues too few
+// registers and take half as long again (75 us against 50 at 32640 pixels), 256-wide ones would leave no
+// tensor memory for t.  The FP32 sums run over K in the same order as in the separate GEMMs and each
+// epilogue applies the same operations in the same order, with x and t rounded to 16 bits where the
+// separate launches stored them, so the result is bitwise theirs.
 #include "dcb_sm100.cuh"
 
 #include "host_util.h"
@@ -711,15 +711,17 @@ bool dcb_tail_supported(int C, int cdc, int cffn, int n1)
             (C == 256 && cffn == 128 && (cdc == 0 || cdc == 128)));
 }
 
-// The kernel's time goes in waves of one tile per pair of SMs, that of the separate launches with M
-// (one B200, inputs rotating through L2, microseconds fused / separate):
-//   (512, 256, 256): M = 4096 22.1 / 18.3, 6240 22.4 / 23.2, 14400 24.9 / 36.8, 22528 (second wave a
-//     fifth full) 47.5 / 46.8, 25600 47.8 / 52.0, 32640 49.7 / 61.2, 38144 68.0 / 72.3, 129600 174 / 242
-//   (256, 256, 256): M = 1560 15.9 / 15.5, 2560 15.6 / 16.1, 14400 16.8 / 28.0, 19200 28.3 / 36.1
-//   (256, 128, 128): M = 390 11.2 / 12.5, 14400 12.7 / 21.4, 19200 20.9 / 26.1, 129600 72.0 / 91.7
+// The kernel's time goes in waves of one tile per pair of SMs, that of the separate launches with M, by a
+// step where the 256 columns of dc.3 and ffn.2 (128-wide tiles of 512) no longer run in one round, at
+// 128 * num_sms / 4 rows (one B200, inputs rotating through L2, microseconds fused / separate):
+//   (512, 256, 256): M = 4736 21.5 / 16.9, 5120 21.5 / 22.5, 14400 23.7 / 35.7, 22528 (second wave a
+//     fifth full) 45.5 / 44.8, 25600 46.2 / 50.3, 32640 48.3 / 59.2, 129600 173 / 215
+//   (256, 256, 256): M = 4736 14.7 / 13.7, 5120 14.7 / 16.4, 14400 16.1 / 26.8, 19200 27.0 / 31.9
+//   (256, 128, 128): M = 2304 11.2 / 9.3, 4736 11.3 / 11.4, 5120 11.3 / 13.7, 14400 12.5 / 20.2, 19200
+//     20.1 / 24.9, 129600 69 / 88
 // and against the one-SM ConvFFN kernel (ffn_sm100.cu; cdc = 0):
-//   (512, 256): M = 390 17.4 / 38.6, 32640 40.0 / 90.9;  (256, 128): M = 390 9.4 / 11.6, 14400 10.7 / 12.6,
-//     37888 19.3 / 19.3, 129600 61.2 / 57.9
+//   (512, 256): M = 390 17.4 / 38.6, 32640 39.5 / 90.9;  (256, 128): M = 390 9.2 / 11.6, 14400 10.3 / 12.6,
+//     37888 19.3 / 19.3, 129600 58 / 58
 bool dcb_tail_preferred(int M, int C, int cdc, int cffn, int n1)
 {
     if (!dcb_tail_supported(C, cdc, cffn, n1)) {
@@ -729,10 +731,10 @@ bool dcb_tail_preferred(int M, int C, int cdc, int cffn, int n1)
     if (cdc == 0) {
         return cffn == 256 || tiles <= 2 * pairs;
     }
-    if (C == 512) {
-        return M >= 6144 && (tiles <= pairs || 8 * tiles >= 10 * pairs);
+    if (C == 512 && tiles > pairs && 8 * tiles < 10 * pairs) {
+        return false;
     }
-    return cffn == 128 || M >= 2048;
+    return 4LL * ((M + kRows - 1) / kRows) > num_sms();
 }
 
 cudaError_t dcb_tail_sm100(int dtype, const DcbTailParams& p, cudaStream_t stream)
