@@ -4,6 +4,7 @@
 #include "dcb_sm100.cuh"
 #include "ffn_sm100.cuh"
 #include "gemm_sm100.cuh"
+#include "host_util.h"
 #include "quant_tables.h"
 
 #include "../../include/dcvc_b200.h"
@@ -255,6 +256,37 @@ int dcvc_conv_ffn(int M, int C, int cffn, const void* x, int ldx, const void* w1
         return kInvalidArgument;
     }
     return cuda_status(e, "dcvc_conv_ffn");
+}
+
+// Two GEMMs beat the one kernel while the second's 64-wide tiles (128 at 512 channels) run in one round (us
+// back to back, one kernel / two launches: (512, 256) M = 1024 16.9 / 7.4, 4736 17.5 / 12.1, 8160 17.9 / 17.8;
+// (256, 128) 1024 9.2 / 5.8, 4736 9.4 / 8.1, 5120 9.4 / 9.7).
+long long dcvc_conv_ffn_workspace(int M, int C, int cffn)
+{
+    if (M <= 0 || !dcb_tail_supported(C, 0, cffn, 4 * cffn) || 4LL * ((M + 127) / 128) > num_sms()) {
+        return 0;
+    }
+    return 2LL * M * cffn;
+}
+
+int dcvc_conv_ffn_ws(int M, int C, int cffn, const void* x, int ldx, const void* w1, const float* b1,
+                     const void* w2, const float* b2, const void* qscale, void* out, int ldo,
+                     void* workspace, long long workspace_bytes, void* stream)
+{
+    auto odd = [](const void* q) { return q == nullptr || (reinterpret_cast<uintptr_t>(q) & 15) != 0; };
+    const long long need = dcvc_conv_ffn_workspace(M, C, cffn);
+    // the GEMMs read the biases in 16-byte pieces; every other check is theirs and the one kernel's alike
+    if (need == 0 || workspace_bytes < need || odd(workspace) || odd(b1) || odd(b2) || odd(x) || odd(out) || odd(w1) ||
+        odd(w2) || (reinterpret_cast<uintptr_t>(qscale) & 15) != 0 || ldx % 8 != 0 || ldo % 8 != 0) {
+        return dcvc_conv_ffn(M, C, cffn, x, ldx, w1, b1, w2, b2, qscale, out, ldo, 0, stream);
+    }
+    const int st = dcvc_conv1x1(DCVC_F16, kEpiQuad, M, 4 * cffn, C, x, ldx, w1, b1, nullptr, 0, nullptr, 0, nullptr, workspace,
+                                cffn, 0, 0, 0, stream);
+    if (st != kOk) {
+        return st;
+    }
+    return dcvc_conv1x1(DCVC_F16, qscale != nullptr ? kEpiBiasResQ : kEpiBiasRes, M, C, cffn, workspace, cffn, w2, b2, x, ldx,
+                        nullptr, 0, qscale, out, ldo, 0, 0, 0, stream);
 }
 
 int dcvc_dcb_tail(int dtype, int M, int C, int cdc, int cffn, const void* a, int lda, const void* x, int ldx,

@@ -154,6 +154,15 @@ int dcvc_conv_ffn(int M, int C, int cffn, const void* x, int ldx, const void* w1
                   const void* w2, const float* b2, const void* qscale, void* out, int ldo,
                   int block_n, void* stream);
 
+/* dcvc_conv_ffn (block_n = 0) with room for the quad output: dcvc_conv_ffn_workspace() bytes at
+ * workspace, 16-byte aligned, in use until the call's work on the stream is done.  Few pixels are then two
+ * GEMM launches, which is faster there; 0 bytes (workspace may be NULL) where the one kernel is.  The
+ * same bits either way.  No counterpart in the reference. */
+long long dcvc_conv_ffn_workspace(int M, int C, int cffn);
+int dcvc_conv_ffn_ws(int M, int C, int cffn, const void* x, int ldx, const void* w1, const float* b1,
+                     const void* w2, const float* b2, const void* qscale, void* out, int ldo,
+                     void* workspace, long long workspace_bytes, void* stream);
+
 /* The part of a DepthConvBlock behind its depthwise 3x3 in one kernel (layers_proxy.cpp:71-101):
  *   y = a . w0^T + b0 + x;  t = quad(y . w1^T + b1);  out = (t . w2^T + b2 + y) [* qscale]
  * with y and t kept on chip.  a [M, cdc] (pitch lda), x, out [M, C] (pitches ldx, ldo; out may be

@@ -89,3 +89,26 @@ def test_residual_pairs(M, Nn, K, dtype, with_q):
     assert bool(torch.isnan(buf[:, :8]).all()) and bool(torch.isnan(buf[:, 8 + Nn:]).all())
     with pytest.raises(N.DcvcError):  # callers cannot ask for it
         ops.conv1x1(a, w, b, epi, res=res, qscale=q, block_n=N.BLOCK_N_PAIR)
+
+
+@pytest.mark.parametrize("M", [1, 127, 390, 1000, 4736, 4737])
+@pytest.mark.parametrize("C,cffn", [(512, 256), (256, 256), (256, 128)])
+@pytest.mark.parametrize("with_q,in_place", [(False, False), (True, False), (False, True)])
+def test_conv_ffn_of_few_pixels(M, C, cffn, with_q, in_place):
+    """ConvFFN as two GEMMs, up to one row tile past its range: bitwise the tail kernel, also in place, and with
+    biases that the GEMMs could not read (the one kernel takes those)."""
+    g = torch.Generator(device="cuda").manual_seed(M + C + cffn)
+    x = torch.randn(M, C, device="cuda", generator=g).half()
+    w1 = (torch.randn(4 * cffn, C, device="cuda", generator=g) * C ** -0.5).half()
+    w2 = (torch.randn(C, cffn, device="cuda", generator=g) * cffn ** -0.5).half()
+    b1, b2 = (torch.randn(n + 1, device="cuda", generator=g)[1:] * 0.1 for n in (4 * cffn, C))
+    q = (torch.rand(C, device="cuda", generator=g) + 0.5).half() if with_q else None
+    ref = ops.dcb_tail(None, x, None, None, w1, b1, w2, b2, qscale=q)
+    odd = torch.empty(C + 1, device="cuda")[1:].copy_(b2)
+    assert odd.data_ptr() % 16 != 0
+    aside = ops.conv_ffn(x, w1, b1, w2, odd, qscale=q)
+    out = ops.conv_ffn(x, w1, b1, w2, b2, qscale=q, out=x if in_place else None)
+    torch.cuda.synchronize()
+    assert N.device_error() == 0
+    assert torch.equal(out.view(torch.int16), ref.view(torch.int16))
+    assert torch.equal(aside.view(torch.int16), ref.view(torch.int16))
