@@ -33,7 +33,8 @@ enum GemmEpilogue : int {
 // 128-wide channel slices with W resident in shared memory, contiguous row ranges per CTA.
 constexpr int kBlockNStream = -1;
 // block_n value selecting the CTA-pair form (cta_group::2, 256 x 256 tiles over two SMs, each
-// staging half of the W tile) of the bias, WSiLU and quad epilogues with 16-bit operands.
+// staging half of the W tile) of the bias, WSiLU and quad epilogues with 16-bit operands; the library
+// takes it by itself too, with the residual epilogues as well (gemm_pair_preferred).
 constexpr int kBlockNPair = -2;
 // block_n value of the quad epilogue with resident activations (quad_sm100.cu): the library's own
 // choice only.
