@@ -390,6 +390,7 @@ __device__ __forceinline__ uint32_t cluster_cta_rank()
 // accesses.
 __device__ __forceinline__ void cluster_sync()
 {
+    __syncwarp();  // the barrier instructions are for converged warps
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
@@ -447,21 +448,40 @@ __device__ __forceinline__ void tma_load_2d_pair(void* dst, const void* tmap, ui
         : "memory");
 }
 
-__device__ __forceinline__ void tmem_alloc_pair(uint32_t* dst_smem, uint32_t ncols)
+// Tensor memory of a CTA pair.  tcgen05.alloc and tcgen05.dealloc with cta_group::2 are made by a warp of each
+// CTA together and act on the tensor memory of both SMs.  Nothing but a barrier of the cluster shows that the
+// other CTA has started, or that it is still there: a CTA that asks for the pair's columns before its peer
+// runs, or leaves while the peer still gives its columns back, has no bound on when (or whether) that operation
+// ends.  With one stream the two CTAs of a cluster start and end within some hundred clocks of each other; with
+// several codecs on the GPU one SM of a pair can be long in reaching the CTA.  Hence pair_begin() and pair_end().
+
+// All threads of both CTAs, once the barriers of the CTA are initialised: the warp of each CTA for which `alloc_warp` holds allocates.
+__device__ __forceinline__ uint32_t pair_begin(uint32_t* dst_smem, uint32_t ncols, bool alloc_warp)
 {
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst_smem)),
-                 "r"(ncols)
-                 : "memory");
+    cluster_sync();  // both CTAs run; their barriers are initialised before any copy or arrive reaches them
+    if (alloc_warp) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst_smem)),
+                     "r"(ncols)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    return *dst_smem;
 }
 
-__device__ __forceinline__ void tmem_relinquish_pair()
+// All threads of both CTAs, last.
+__device__ __forceinline__ void pair_end(uint32_t taddr, uint32_t ncols, bool alloc_warp)
 {
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-}
-
-__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols)
-{
-    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();  // both CTAs are done with the pair's accumulators and each other's barriers
+    if (alloc_warp) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+    }
+    cluster_sync();  // and have both given the columns back
 }
 
 // M = 256 MMA over both CTAs' operands (issued by the even CTA).

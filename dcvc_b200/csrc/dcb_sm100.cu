@@ -174,15 +174,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         *abort_flag = 0;
         fence_mbar_init();
     }
-    if (warp == 1) {
-        tmem_alloc_pair(tmem_slot, kTmemCols);
-        tmem_relinquish_pair();
-    }
-    tc_fence_before();
-    __syncthreads();
-    cluster_sync();  // the peer's barriers are initialised before any copy or arrive reaches them
-    tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = pair_begin(tmem_slot, kTmemCols, warp == 1);
     griddep_launch_dependents();
     griddep_wait();
 
@@ -662,13 +654,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
     }
 
-    tc_fence_before();
-    __syncthreads();
-    cluster_sync();  // both CTAs are done with the pair's accumulators and each other's barriers
-    if (warp == 1) {
-        tc_fence_after();
-        tmem_dealloc_pair(tmem_base, kTmemCols);
-    }
+    pair_end(tmem_base, kTmemCols, warp == 1);
 }
 
 template <typename T, int C, int K0, int F>

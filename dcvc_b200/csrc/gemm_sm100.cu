@@ -194,22 +194,19 @@ __global__ void __launch_bounds__(GemmCfg<BN, EPI, PAIR>::kThreads, 1)
         tma_prefetch_desc(&tmA);
         tma_prefetch_desc(&tmB);
     }
-    if (warp == 1) {
-        if constexpr (PAIR) {
-            tmem_alloc_pair(tmem_slot, C::kTmemCols);
-            tmem_relinquish_pair();
-        } else {
+    uint32_t tmem_base;
+    if constexpr (PAIR) {
+        tmem_base = pair_begin(tmem_slot, C::kTmemCols, warp == 1);
+    } else {
+        if (warp == 1) {
             tmem_alloc(tmem_slot, C::kTmemCols);
             tmem_relinquish();
         }
+        tc_fence_before();
+        __syncthreads();
+        tc_fence_after();
+        tmem_base = *tmem_slot;
     }
-    tc_fence_before();
-    __syncthreads();
-    if constexpr (PAIR) {
-        cluster_sync();  // the peer's barriers are initialised before any copy or arrive reaches them
-    }
-    tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
     // A small GEMM is a chain of latencies (4 us, of which its MMAs run for one).  The first tile's place
     // is found before the wait: its divisions and first reads of the parameters held the first copy up by
     // 500 clocks.  With the bias loaded ahead and the look at the next stage (below): 1024 x 384 x 384 bias
@@ -716,17 +713,13 @@ __global__ void __launch_bounds__(GemmCfg<BN, EPI, PAIR>::kThreads, 1)
         __syncwarp();
     }
 
-    tc_fence_before();
-    __syncthreads();
     if constexpr (PAIR) {
-        // both CTAs are done with the pair's accumulators and with each other's barriers
-        cluster_sync();
-    }
-    if (warp == 1) {
-        tc_fence_after();
-        if constexpr (PAIR) {
-            tmem_dealloc_pair(tmem_base, C::kTmemCols);
-        } else {
+        pair_end(tmem_base, C::kTmemCols, warp == 1);
+    } else {
+        tc_fence_before();
+        __syncthreads();
+        if (warp == 1) {
+            tc_fence_after();
             tmem_dealloc(tmem_base, C::kTmemCols);
         }
     }
