@@ -136,17 +136,29 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
     return true;
 }
 
-// One look at a barrier, without waiting.
+// One look at a barrier, without waiting (CLUSTER: one that also receives arrivals of the other CTA of a pair,
+// acquired at cluster scope).
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity)
 {
     uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
+    if constexpr (CLUSTER) {
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(smem_u32(bar)), "r"(parity)
+            : "memory");
+    } else {
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(smem_u32(bar)), "r"(parity)
+            : "memory");
+    }
     return ok != 0;
 }
 
@@ -402,12 +414,6 @@ __device__ __forceinline__ uint32_t cluster_map(const void* p, uint32_t rank)
     return r;
 }
 
-// Arrive on an mbarrier of another CTA of the cluster (address from cluster_map).
-__device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr)
-{
-    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-
 // Predicated forms: a branch around one lane's instruction costs its warp some hundred clocks.
 __device__ __forceinline__ void mbar_arrive_if(bool pred, uint64_t* bar)
 {
@@ -417,14 +423,40 @@ __device__ __forceinline__ void mbar_arrive_if(bool pred, uint64_t* bar)
                  : "memory");
 }
 
-// `n` arrivals at once on a barrier of any CTA of the cluster (address from cluster_map).
-__device__ __forceinline__ void mbar_arrive_remote_if(bool pred, uint32_t cluster_addr, uint32_t n)
+// Arrivals of a pair's CTAs on a barrier of the even one, which its MMA warp waits for with acquire at cluster
+// scope.  Without a scope an arrival orders nothing outside its own CTA, so each says what crosses:
+//
+// Tensor memory alone (an accumulator has been read, values have been written to it): the loads and stores are
+// complete (tcgen05.wait) and tcgen05.fence::before_thread_sync orders them before the arrival, ::after_thread_sync
+// the MMA behind the wait.  No other memory is involved, so the arrival itself need not release any: relaxed, at
+// cluster scope.  `n` arrivals at once (address from cluster_map).
+__device__ __forceinline__ void mbar_arrive_tmem_if(bool pred, uint32_t cluster_addr, uint32_t n)
 {
     asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p mbarrier.arrive.shared::cluster.b64 _, [%0], %1;\n\t}" ::"r"(
-            cluster_addr),
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t"
+        "@p mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0], %1;\n\t}" ::"r"(cluster_addr),
         "r"(n), "r"(static_cast<int>(pred))
         : "memory");
+}
+
+// Shared memory (the odd CTA's part of an operand that the MMA reads from both CTAs): a release at cluster scope.  It
+// waits for all that its thread has in flight, and the next step of the MMA warp waits for it (tail kernel, us at
+// 32640 pixels and 512 channels: 49.2 without an order between the CTAs, 65.4 with a release in every arrival, 51.6
+// with one per warp and 64 columns of x, 51.0 as here).  So the writing warps arrive on a barrier of their own CTA,
+// and one warp that has nothing in flight, the odd CTA's idle MMA warp, waits for it and arrives once, for all of
+// them, on the even CTA's barrier at the same place, which counts the even CTA's warps and that one arrival.
+// `even`: the distance from this CTA's shared memory to the even CTA's.
+__device__ __forceinline__ bool pair_pass(uint64_t* bar, uint32_t parity, uint32_t even, long long limit_cycles)
+{
+    if (!mbar_wait_warp(bar, parity, limit_cycles)) {
+        return false;
+    }
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %1, 0;\n\t"
+        "@p mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n\t}" ::"r"(smem_u32(bar) + even),
+        "r"(static_cast<int>(elect_one()))
+        : "memory");
+    return true;
 }
 
 __device__ __forceinline__ void tma_store_2d_if(bool pred, const void* tmap, uint32_t src, int c0, int c1)

@@ -96,7 +96,8 @@ struct TailCfg {
     static constexpr int kBiasOffset = kBarOffset + kBarBytes;
     static constexpr int kBytes = kBiasOffset + kBiasBytes + 1024;
     static constexpr int kTStages = F / 128;
-    static constexpr int kBars = 2 * kStages + 2 * kAccs + 2 + kASlabs + 3 * kXSlabs + kTStages;
+    static constexpr int kXStages = C / 128;     // 128 columns of x: what one stage of ffn.0 reads
+    static constexpr int kBars = 2 * kStages + 2 * kAccs + 2 + kASlabs + kXStages + 2 * kXSlabs + kTStages;
     static_assert((C == 256 || C == 512) && K0 % 128 == 0 && (F == 128 || F == 256), "channel counts");
     static_assert(kAccCol >= F / 2 && kAccCol + kAccs * kNB <= kTmemCols, "tensor memory");
     static_assert(K0 == 0 || kOwnA || 2 * K0 <= C, "dc.3 operand in the upper half of x");
@@ -134,8 +135,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     uint64_t* adone = accempty + kAccs;      // dc.3's MMAs of a tile have read the operand
     uint64_t* drain = adone + 1;
     uint64_t* afull = drain + 1;           // E: operand slab landed in both CTAs
-    uint64_t* xfull = afull + G::kASlabs;  // E: x slab complete in both CTAs
-    uint64_t* xfree = xfull + G::kXSlabs;  // output stored from the slab
+    uint64_t* xfull = afull + G::kASlabs;  // E: 128 columns of x complete in both CTAs (cdc > 0: see pair_pass)
+    uint64_t* xfree = xfull + G::kXStages; // output stored from the slab
     uint64_t* tfull = xfree + G::kXSlabs;  // E: 128 values of t complete in both CTAs
     uint64_t* rfull = tfull + G::kTStages; // residual slab landed
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(rfull + G::kXSlabs);
@@ -165,8 +166,11 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
         for (int s = 0; s < G::kXSlabs; ++s) {
             mbar_init(&rfull[s], 1);
-            mbar_init(&xfull[s], K0 > 0 ? 8 : 1);  // the four quadrants' warps of both CTAs, or the copies
             mbar_init(&xfree[s], 4);
+        }
+        for (int b = 0; b < G::kXStages; ++b) {
+            // the four quadrants' warps of two slabs and the odd CTA's arrival for all of its, or two copies
+            mbar_init(&xfull[b], K0 > 0 ? 8 + (rank == 0 ? 1 : 0) : 2);
         }
         for (int b = 0; b < G::kTStages; ++b) {
             mbar_init(&tfull[b], 4 * 2 * kEpiWarps);  // four blocks of ffn.0
@@ -334,10 +338,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 for (int i = 0; ok && i < G::kBlocksT; ++i) {
                     ok = begin();
                     for (int kb = 0; ok && kb < C / 128; ++kb) {
-                        for (int t = 0; ok && i == 0 && t < kStageTiles; ++t) {
-                            ok = need(&xfull[kb * kStageTiles + t], tp);
-                        }
-                        ok = ok && kblock(0, kb);
+                        ok = (i > 0 || need(&xfull[kb], tp)) && kblock(0, kb);
                     }
                     if (ok) {
                         finish();
@@ -359,6 +360,16 @@ __global__ void __launch_bounds__(kThreads, 1)
                 }
                 __syncwarp();
                 mbar_wait_warp(drain, 0, kWaitLimit / 16);
+            }
+        } else if constexpr (K0 > 0) {
+            // ---------------------------------------------------- the odd CTA's x, told to the even CTA
+            const uint32_t even = cluster_map(smem, 0) - smem_u32(smem);
+            bool ok = true;
+            uint32_t tp = 0;
+            for (int tile = unit; ok && tile < num_tiles && !warp_any(*abort_flag != 0); tile += units, tp ^= 1) {
+                for (int b = 0; ok && b < G::kXStages; ++b) {
+                    ok = pair_pass(&xfull[b], tp, even, kWaitLimit) || fail(kErrGemmMmaTimeout);
+                }
             }
         }
     } else if (warp == 2) {
@@ -408,7 +419,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 for (int s = 0; ok && s < G::kXSlabs; ++s) {
                     ok = gate(&xfree[s], tp ^ 1);
                     if (ok) {
-                        load(&tmX, &xfull[s], s, s * 64, m0);
+                        load(&tmX, &xfull[s / 2], s, s * 64, m0);
                     }
                 }
             } else if constexpr (G::kOwnA) {
@@ -461,7 +472,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
         if (warp_any(*abort_flag != 0) && rank == 0) {
             // let the copies that count on this CTA's barriers land before it winds down
-            for (int s = 0; s < (K0 > 0 ? G::kASlabs : G::kXSlabs); ++s) {
+            for (int s = 0; s < (K0 > 0 ? G::kASlabs : G::kXStages); ++s) {
                 mbar_wait_warp(K0 > 0 ? &afull[s] : &xfull[s], tp, kWaitLimit / 16);
             }
         }
@@ -476,9 +487,9 @@ __global__ void __launch_bounds__(kThreads, 1)
         const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
         int acc = 0;
         uint32_t acc_phase = 0;
-        // `n` arrivals on a barrier of the even CTA, after a __syncwarp
+        // arrivals on a barrier of the even CTA, after a __syncwarp
         const uint32_t even = cluster_map(smem, 0) - smem_u32(smem);
-        auto arrive_even = [&](uint64_t* bar, uint32_t n) { mbar_arrive_remote_if(lane == 0, smem_u32(bar) + even, n); };
+        auto arrive_tmem = [&](uint64_t* bar, uint32_t n) { mbar_arrive_tmem_if(lane == 0, smem_u32(bar) + even, n); };
         auto advance = [&] {
             if (++acc == kAccs) {
                 acc = 0;
@@ -507,7 +518,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         auto release_acc = [&](uint32_t n) {
             tc_fence_before();
             __syncwarp();
-            arrive_even(&accempty[acc], n);
+            arrive_tmem(&accempty[acc], n);
             advance();
         };
         auto load_acc = [&](uint32_t (&r)[32], int col) {
@@ -595,7 +606,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                         break;
                     }
                     residual_slab(s, s * 64, std::false_type{}, nullptr);
-                    arrive_even(&xfull[s], 1);
+                    mbar_arrive_if(lane == 0, &xfull[s / 2]);
                 }
             }
             // ffn.0: 32 columns -> 8 values of t per row, to tensor memory
@@ -621,7 +632,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 tc_wait_st();
                 tc_fence_before();
                 __syncwarp();
-                arrive_even(&tfull[nb / 4], 1);
+                arrive_tmem(&tfull[nb / 4], 1);
             }
             // ffn.2: out = (acc + b2 + x) [* q], over x in its slab and stored from there
 #pragma unroll 1

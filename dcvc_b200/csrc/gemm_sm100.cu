@@ -313,7 +313,7 @@ __global__ void __launch_bounds__(GemmCfg<BN, EPI, PAIR>::kThreads, 1)
             bool ok = true;
             bool ready = false;  // the stage's copies were seen complete before the loop came round
             for (int tile = unit; ok && tile < num_tiles && !warp_any(*abort_flag != 0); tile += units) {
-                if (!mbar_wait_warp(&tempty[acc], acc_phase ^ 1, lim)) {
+                if (!mbar_wait_warp<PAIR>(&tempty[acc], acc_phase ^ 1, lim)) {
                     ok = fail(kErrGemmMmaTimeout);
                     break;
                 }
@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(GemmCfg<BN, EPI, PAIR>::kThreads, 1)
                 const uint32_t d = tmem_base + static_cast<uint32_t>(acc * BN);
                 for (int kb = 0; kb < kblocks; kb += per) {
                     const int tiles = min(per, kblocks - kb);
-                    if (!ready && !mbar_wait_warp(&full[stage], phase, lim)) {
+                    if (!ready && !mbar_wait_warp<PAIR>(&full[stage], phase, lim)) {
                         ok = fail(kErrGemmMmaTimeout);
                         break;
                     }
@@ -366,7 +366,7 @@ __global__ void __launch_bounds__(GemmCfg<BN, EPI, PAIR>::kThreads, 1)
                         }
                         // The warp comes back together when the last MMA above has left the queue; the
                         // wait for the next stage would then cost its latency between two MMAs.
-                        next_ready = mbar_test(&full[next], next_phase);
+                        next_ready = mbar_test<PAIR>(&full[next], next_phase);
                     }
                     ready = warp_any(next_ready);
                     issued_any = true;
@@ -683,12 +683,10 @@ __global__ void __launch_bounds__(GemmCfg<BN, EPI, PAIR>::kThreads, 1)
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) {
-                if (PAIR && rank != 0) {
-                    mbar_arrive_remote(cluster_map(&tempty[acc], 0));  // the even CTA's barrier
-                } else {
-                    mbar_arrive(&tempty[acc]);
-                }
+            if constexpr (PAIR) {
+                mbar_arrive_tmem_if(lane == 0, cluster_map(&tempty[acc], 0), 1);  // the even CTA's barrier
+            } else if (lane == 0) {
+                mbar_arrive(&tempty[acc]);
             }
             acc ^= 1;
             if (acc == 0) {

@@ -362,7 +362,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 if (c == 1) {
                     tc_fence_before();
                     __syncwarp();
-                    mbar_arrive_remote_if(lane == 0, smem_u32(&accempty[acc]) + even, 1);
+                    mbar_arrive_tmem_if(lane == 0, smem_u32(&accempty[acc]) + even, 1);
                 }
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
