@@ -23,6 +23,7 @@
 // separate launches stored them, so the result is bitwise theirs.
 #include "dcb_sm100.cuh"
 
+#include "gemm_sm100.cuh"
 #include "host_util.h"
 
 #include <cstring>
@@ -149,6 +150,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int unit = static_cast<int>(blockIdx.x >> 1);
     const int units = static_cast<int>(gridDim.x >> 1);
     const int row_off = static_cast<int>(rank) * kRows;
+    // progress waits give up after `lim` cycles; the drains after an abort keep the full limit
+    const long long lim = p.wait_limit > 0 ? p.wait_limit : kWaitLimit;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) {
@@ -195,7 +198,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         int issued = 0;
         // K columns 128 kb .. of block nb's weight rows: this CTA's half of them
         auto push = [&](const CUtensorMap* tm, int kb, int nb) {
-            if (!mbar_wait_warp(&wempty[stage], phase ^ 1, kWaitLimit)) {
+            if (!mbar_wait_warp(&wempty[stage], phase ^ 1, lim)) {
                 return fail(kErrGemmProducerTimeout);
             }
             if (elect_one()) {
@@ -258,7 +261,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             uint32_t acc_phase = 0;
             bool issued_any = false;
             auto need = [&](uint64_t* bar, uint32_t parity) {
-                if (!mbar_wait_warp<true>(bar, parity, kWaitLimit)) {
+                if (!mbar_wait_warp<true>(bar, parity, lim)) {
                     return fail(kErrGemmMmaTimeout);
                 }
                 tc_fence_after();
@@ -315,7 +318,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                     acc_phase ^= 1;
                 }
             };
-            bool ok = true;
+            bool ok = p.stall_test == 0;
             uint32_t tp = 0;  // parity of the per-tile barriers
             for (int tile = unit; ok && tile < num_tiles && !warp_any(*abort_flag != 0); tile += units, tp ^= 1) {
                 if constexpr (K0 > 0) {
@@ -368,7 +371,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             uint32_t tp = 0;
             for (int tile = unit; ok && tile < num_tiles && !warp_any(*abort_flag != 0); tile += units, tp ^= 1) {
                 for (int b = 0; ok && b < G::kXStages; ++b) {
-                    ok = pair_pass(&xfull[b], tp, even, kWaitLimit) || fail(kErrGemmMmaTimeout);
+                    ok = pair_pass(&xfull[b], tp, even, lim) || fail(kErrGemmMmaTimeout);
                 }
             }
         }
@@ -376,17 +379,25 @@ __global__ void __launch_bounds__(kThreads, 1)
         // ------------------------------------------------------------ activation slabs
         uint32_t tp = 0;
         auto gate = [&](uint64_t* bar, uint32_t parity) {
-            return mbar_wait_warp(bar, parity, kWaitLimit) || fail(kErrGemmProducerTimeout);
+            return mbar_wait_warp(bar, parity, lim) || fail(kErrGemmProducerTimeout);
         };
-        // operand (afull) or ConvFFN input (xfull) slab of both CTAs
-        auto load = [&](const CUtensorMap* tm, uint64_t* bar, int slab, int c, int m0) {
+        // the barriers on which copies have been asked for, one bit each, and the parity of the last of them: what
+        // has to land before the CTA winds down after an abort
+        uint32_t copies = 0, copies_parity = 0, residuals = 0, residuals_parity = 0;
+        auto note = [](uint32_t& set, uint32_t& par, int bit, uint32_t parity) {
+            set |= 1u << bit;
+            par = (par & ~(1u << bit)) | parity << bit;
+        };
+        // operand (afull) or ConvFFN input (xfull) slab of both CTAs, on barrier `i` of `bars`
+        auto load = [&](const CUtensorMap* tm, uint64_t* bars, int i, uint32_t parity, int slab, int c, int m0) {
             if (elect_one()) {
                 if (rank == 0) {
-                    mbar_arrive_expect_tx(bar, 2 * kSlabBytes);
+                    mbar_arrive_expect_tx(&bars[i], 2 * kSlabBytes);
                 }
-                tma_load_2d_pair(smem + slab * kSlabBytes, tm, cluster_map(bar, 0), c, m0);
+                tma_load_2d_pair(smem + slab * kSlabBytes, tm, cluster_map(&bars[i], 0), c, m0);
             }
             __syncwarp();
+            note(copies, copies_parity, i, parity);
         };
         auto prefetch = [&](const CUtensorMap* tm, int slabs, int m0) {
             if (elect_one()) {
@@ -396,19 +407,18 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
             __syncwarp();
         };
-        uint32_t residuals = 0;  // slabs whose residual has been asked for (drained after an abort)
         auto load_residual = [&](int s, int m0) {
             if (elect_one()) {
                 mbar_arrive_expect_tx(&rfull[s], kSlabBytes);
                 tma_load_2d(smem + s * kSlabBytes, &tmX, &rfull[s], s * 64, m0);
             }
             __syncwarp();
-            residuals |= 1u << s;
+            note(residuals, residuals_parity, s, tp);
         };
         bool ok = true;
         if constexpr (G::kOwnA) {
             for (int s = 0; s < G::kASlabs; ++s) {
-                load(&tmA, &afull[s], G::kAFirst + s, s * 64, unit * 2 * kRows + row_off);
+                load(&tmA, afull, s, 0, G::kAFirst + s, s * 64, unit * 2 * kRows + row_off);
             }
         }
         for (int tile = unit; tile < num_tiles && ok && !warp_any(*abort_flag != 0); tile += units, tp ^= 1) {
@@ -419,7 +429,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 for (int s = 0; ok && s < G::kXSlabs; ++s) {
                     ok = gate(&xfree[s], tp ^ 1);
                     if (ok) {
-                        load(&tmX, &xfull[s / 2], s, s * 64, m0);
+                        load(&tmX, xfull, s / 2, tp, s, s * 64, m0);
                     }
                 }
             } else if constexpr (G::kOwnA) {
@@ -432,14 +442,14 @@ __global__ void __launch_bounds__(kThreads, 1)
                 if (more && ok) {
                     ok = gate(adone, tp);
                     for (int s = 0; ok && s < G::kASlabs; ++s) {
-                        load(&tmA, &afull[s], G::kAFirst + s, s * 64, m1);
+                        load(&tmA, afull, s, tp ^ 1, G::kAFirst + s, s * 64, m1);
                     }
                 }
             } else {
                 for (int s = 0; ok && s < G::kASlabs; ++s) {
                     ok = gate(&xfree[G::kAFirst + s], tp ^ 1);
                     if (ok) {
-                        load(&tmA, &afull[s], G::kAFirst + s, s * 64, m0);
+                        load(&tmA, afull, s, tp, G::kAFirst + s, s * 64, m0);
                     }
                 }
                 if (tile == unit) {
@@ -464,16 +474,14 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
         }
         if (warp_any(*abort_flag != 0)) {
+            // let the copies land before the CTA winds down (those into both CTAs count on the even one's barriers)
             for (int s = 0; s < G::kXSlabs; ++s) {
                 if ((residuals >> s) & 1u) {
-                    mbar_wait_warp(&rfull[s], tp, kWaitLimit / 16);
+                    mbar_wait_warp(&rfull[s], (residuals_parity >> s) & 1u, kWaitLimit / 16);
                 }
-            }
-        }
-        if (warp_any(*abort_flag != 0) && rank == 0) {
-            // let the copies that count on this CTA's barriers land before it winds down
-            for (int s = 0; s < (K0 > 0 ? G::kASlabs : G::kXStages); ++s) {
-                mbar_wait_warp(K0 > 0 ? &afull[s] : &xfull[s], tp, kWaitLimit / 16);
+                if (rank == 0 && ((copies >> s) & 1u)) {
+                    mbar_wait_warp(K0 > 0 ? &afull[s] : &xfull[s], (copies_parity >> s) & 1u, kWaitLimit / 16);
+                }
             }
         }
     } else {
@@ -508,7 +516,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         uint32_t bias_addr;  // known from here on: reads of the biases cannot move above the barrier
         asm volatile("mov.u32 %0, %1;" : "=r"(bias_addr) : "r"(smem_u32(bias)) : "memory");
         auto wait_acc = [&] {
-            if (!mbar_wait_warp(&accfull[acc], acc_phase, kWaitLimit)) {
+            if (!mbar_wait_warp(&accfull[acc], acc_phase, lim)) {
                 return fail(kErrGemmEpilogueTimeout);
             }
             tc_fence_after();
@@ -597,7 +605,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                         continue;
                     }
                     const int s = nb * 2 + side;
-                    if (!mbar_wait_warp(&rfull[s], tp, kWaitLimit)) {
+                    if (!mbar_wait_warp(&rfull[s], tp, lim)) {
                         ok = fail(kErrGemmEpilogueTimeout);
                         break;
                     }
@@ -734,8 +742,10 @@ bool dcb_tail_preferred(int M, int C, int cdc, int cffn, int n1)
     return 4LL * ((M + kRows - 1) / kRows) > num_sms();
 }
 
-cudaError_t dcb_tail_sm100(int dtype, const DcbTailParams& p, cudaStream_t stream)
+cudaError_t dcb_tail_sm100(int dtype, const DcbTailParams& p_in, cudaStream_t stream)
 {
+    DcbTailParams p = p_in;
+    p.stall_test = gemm_take_stall(&p.wait_limit) ? 1 : 0;
     auto bad = [](const void* q) { return q == nullptr || (reinterpret_cast<uintptr_t>(q) & 15) != 0; };
     if (p.M <= 0 || (dtype != 0 && dtype != 1) || !dcb_tail_supported(p.C, p.cdc, p.cffn, 4 * p.cffn) || bad(p.x) ||
         p.ldx % 8 != 0 || bad(p.out) || p.ldo % 8 != 0 || bad(p.w1) || bad(p.w2) || p.b1 == nullptr || p.b2 == nullptr ||

@@ -26,6 +26,10 @@ struct DcbTailParams {
     void* out;            // [M, C], pitch ldo
     int ldo;
     int* err;             // device error word
+    // Test hook (gemm_inject_stall; 0 in production): the MMA warp issues nothing, so every wait behind it runs out
+    // after wait_limit cycles (0: the kernel's own limit, ~1 s) and the drains find copies that have landed.
+    int stall_test;
+    long long wait_limit;
 };
 
 // Whether dcb_tail_sm100 has a form for these channel counts (n1 = ffn.0 output channels, cdc = 0:

@@ -857,15 +857,22 @@ void gemm_inject_stall(int launches, long long wait_limit_cycles)
     g_stall_launches.store(launches > 0 ? launches : 0);
 }
 
-GemmParams gemm_apply_injection(const GemmParams& p)
+bool gemm_take_stall(long long* wait_limit_cycles)
 {
-    GemmParams q = p;
     int n = g_stall_launches.load();
     while (n > 0 && !g_stall_launches.compare_exchange_weak(n, n - 1)) {
     }
     if (n > 0) {
+        *wait_limit_cycles = g_stall_limit.load();
+    }
+    return n > 0;
+}
+
+GemmParams gemm_apply_injection(const GemmParams& p)
+{
+    GemmParams q = p;
+    if (gemm_take_stall(&q.wait_limit)) {
         q.stall_test = 1;
-        q.wait_limit = g_stall_limit.load();
     }
     return q;
 }

@@ -82,6 +82,8 @@ struct GemmParams {
 // The next `launches` GEMM launches of this process run with stall_test set and the given wait
 // limit (failure-detection tests; launches <= 0 cancels).
 void gemm_inject_stall(int launches, long long wait_limit_cycles);
+// Takes one pending injection: true, and its wait limit, if there was one.
+bool gemm_take_stall(long long* wait_limit_cycles);
 // Applies a pending injection to a launch's parameters (used by the GEMM launchers).
 GemmParams gemm_apply_injection(const GemmParams& p);
 
