@@ -13,7 +13,7 @@ namespace dcvc {
 cudaError_t gemm_autotune(int dtype, int epi, const GemmParams& shape, cudaStream_t stream,
                           int* best_bn, float* best_us);
 void gemm_autotune_set_enabled(bool on);
-int gemm_tuned_bn(int dtype, int epi, int M, int N, int K, int sub_w);
+int gemm_recorded_bn(int dtype, int epi, int M, int N, int K, int sub_w);
 void gemm_tuning_clear();
 cudaError_t gemm_sm100(int dtype, const void* A, int lda, const void* W, const GemmParams& p,
                        int epi, int bn, cudaStream_t stream);
@@ -121,7 +121,7 @@ int dcvc_conv1x1_f8(int epilogue, int M, int N, int K, const void* a, int lda, c
     p.out = out;
     p.ldo = ldo;
     p.err = device_error_word();
-    cudaError_t e = block_n == kBlockNResident
+    cudaError_t e = block_n <= kBlockNResident
                         ? cudaErrorInvalidValue
                         : gemm_sm100(kDtypeF8, a, lda, w, p, epilogue, block_n, static_cast<cudaStream_t>(stream));
     if (e == cudaErrorInvalidValue) {
@@ -178,7 +178,7 @@ int dcvc_conv1x1(int dtype, int epilogue, int M, int N, int K, const void* a, in
     p.sub_w = sub_w;
     p.sub_cout = sub_cout;
     p.err = device_error_word();
-    cudaError_t e = block_n == kBlockNResident
+    cudaError_t e = block_n <= kBlockNResident
                         ? cudaErrorInvalidValue
                         : gemm_sm100(dtype, a, lda, w, p, epilogue, block_n, static_cast<cudaStream_t>(stream));
     if (e == cudaErrorInvalidValue) {
@@ -226,7 +226,7 @@ int dcvc_gemm_tuned(int dtype, int epilogue, int M, int N, int K, int sub_w, int
         set_last_error("dcvc_gemm_tuned: null output");
         return kInvalidArgument;
     }
-    *block_n = gemm_tuned_bn(dtype, epilogue, M, N, K, epilogue == kEpiSubpel ? sub_w : 0);
+    *block_n = gemm_recorded_bn(dtype, epilogue, M, N, K, epilogue == kEpiSubpel ? sub_w : 0);
     return kOk;
 }
 

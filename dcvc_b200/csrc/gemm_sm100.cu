@@ -917,13 +917,10 @@ cudaError_t gemm_sm100(int dtype, const void* A, int lda, const void* W, const G
                (epi != kEpiBias && epi != kEpiBiasWsilu && epi != kEpiQuad))) {
         return cudaErrorInvalidValue;
     }
-    const bool chosen = bn == 0;
+    const bool chosen = bn == 0 || bn == kBlockNRule;
     if (chosen) {
-        // a width measured by the autotuner (gemm_tune.cu) for this shape, else the rule
-        bn = gemm_tuned_bn(dtype, epi, p.M, p.N, p.K, epi == kEpiSubpel ? p.sub_w : 0);
-        if (epi == kEpiQuad) {
-            bn = 0;  // one width is recorded for this epilogue, the forms of it are the rule's
-        }
+        // a width that the autotuner (gemm_tune.cu) measured to be faster than the rule for this shape, else the rule
+        bn = bn == 0 ? gemm_tuned_bn(dtype, epi, p.M, p.N, p.K, epi == kEpiSubpel ? p.sub_w : 0) : 0;
         if (bn == 0) {
             bn = gemm_pick_bn(p.M, p.N, epi, p.sub_cout, p.K);
             if (epi == kEpiQuad && bn > 0) {

@@ -39,6 +39,8 @@ constexpr int kBlockNPair = -2;
 // block_n value of the quad epilogue with resident activations (quad_sm100.cu): the library's own
 // choice only.
 constexpr int kBlockNResident = -3;
+// The rule's choice whatever the autotuner has recorded (gemm_tune.cu measures it).
+constexpr int kBlockNRule = -4;
 
 struct GemmParams {
     int M, N, K;

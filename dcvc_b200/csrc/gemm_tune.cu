@@ -3,13 +3,14 @@
 // The reference picks a CUTLASS configuration per layer shape from compile-time tables filled
 // offline per GPU (HINT_MAP_* in cutlass/conv1x1_bias.cu:8 and its siblings, looked up by
 // launch_cutlass_helper, cutlass/cutlass_kernel.h:232-250, with a default hint for shapes not
-// in the table).  Here the choice is the N tile width of the tcgen05 kernel (256, 128 or 64),
-// measured at run time: gemm_autotune() times every valid width for one shape on scratch
-// operands with CUDA events and records the fastest in a process-wide table keyed by (dtype,
-// epilogue, M, N, K, sub_w); gemm_sm100 consults the table whenever the caller leaves the width
-// to the library, and falls back to gemm_pick_bn's rule for untuned shapes.  The tile width
-// never changes an output bit (every output element is one accumulator column reduced over K in
-// the same order), so tuning affects speed only.
+// in the table).  Here the choice is a rule on the shape (gemm_sm100.cu: tile widths of 256 to 32, CTA pairs,
+// the streaming form, resident activations), and gemm_autotune() measures at run time whether a fixed width
+// beats it: it times the rule's own choice, the tile widths 256, 128 and 64 and, where it exists, the streaming
+// form for one shape on scratch operands with CUDA events, and records the fastest width in a process-wide
+// table keyed by (device, dtype, epilogue, M, N, K, sub_w).  gemm_sm100 takes a recorded width, when the caller
+// leaves the width to the library, only if it was faster than the rule.  The form never changes an output bit
+// (every output element is one accumulator column reduced over K in the same order), so tuning affects speed
+// only.
 //
 // Tuning allocates and frees device memory and synchronises the stream, so it never runs while
 // the stream is being captured into a graph: the codecs tune a shape on the first, eager
@@ -56,6 +57,7 @@ int current_device()
 struct TuneEntry {
     int bn;
     float us;
+    bool beats_rule;
 };
 
 std::mutex g_tune_mu;
@@ -64,6 +66,7 @@ std::atomic<size_t> g_tuned_count{0};  // lets untuned processes skip the lock
 std::atomic<int> g_enabled{-1};  // -1: not read from the environment yet
 
 constexpr int kTuneReps = 5;
+constexpr float kTuneMargin = 0.97f;  // a width has to be faster than the rule's form by more than the noise of a run
 
 bool epi_has_res(int e) { return e == kEpiBiasRes || e == kEpiBiasResQ || e == kEpiBiasRes2; }
 
@@ -105,15 +108,44 @@ bool gemm_autotune_enabled()
 
 void gemm_autotune_set_enabled(bool on) { g_enabled.store(on ? 1 : 0); }
 
-int gemm_tuned_bn(int dtype, int epi, int M, int N, int K, int sub_w)
+namespace {
+
+bool find_tuned(int dtype, int epi, int M, int N, int K, int sub_w, TuneEntry* out)
 {
     if (g_tuned_count.load(std::memory_order_acquire) == 0) {
-        return 0;
+        return false;
     }
     const int dev = current_device();
     std::lock_guard<std::mutex> lk(g_tune_mu);
     auto it = g_tuned.find(TuneKey{dev, dtype, epi, M, N, K, sub_w});
-    return it == g_tuned.end() ? 0 : it->second.bn;
+    if (it == g_tuned.end()) {
+        return false;
+    }
+    *out = it->second;
+    return true;
+}
+
+void record_tuned(int dtype, int epi, const GemmParams& p, const TuneEntry& e)
+{
+    std::lock_guard<std::mutex> lk(g_tune_mu);
+    g_tuned[TuneKey{current_device(), dtype, epi, p.M, p.N, p.K, epi == kEpiSubpel ? p.sub_w : 0}] = e;
+    g_tuned_count.store(g_tuned.size(), std::memory_order_release);
+}
+
+}  // namespace
+
+// The recorded width of a shape, whether or not it is used (0: none recorded).
+int gemm_recorded_bn(int dtype, int epi, int M, int N, int K, int sub_w)
+{
+    TuneEntry e;
+    return find_tuned(dtype, epi, M, N, K, sub_w, &e) ? e.bn : 0;
+}
+
+// The recorded width if it was measured faster than the rule's own choice, else 0.
+int gemm_tuned_bn(int dtype, int epi, int M, int N, int K, int sub_w)
+{
+    TuneEntry e;
+    return find_tuned(dtype, epi, M, N, K, sub_w, &e) && e.beats_rule ? e.bn : 0;
 }
 
 void gemm_tuning_clear()
@@ -123,7 +155,7 @@ void gemm_tuning_clear()
     g_tuned_count.store(0, std::memory_order_release);
 }
 
-// Times every valid N tile width of one shape and records the fastest.  p supplies the shape
+// Times every valid N tile width of one shape and the rule's choice, and records the fastest width.  p supplies the shape
 // (M, N, K, sub_w, sub_cout) only; the operands are zero-filled scratch buffers.  Returns
 // cudaErrorInvalidValue for shapes no width supports and cudaErrorStreamCaptureUnsupported while
 // `stream` is capturing.
@@ -142,8 +174,8 @@ cudaError_t gemm_autotune(int dtype, int epi, const GemmParams& shape, cudaStrea
     if (M <= 0 || N <= 0 || K <= 0) {
         return cudaErrorInvalidValue;
     }
-    int cands[4];
-    int nc = 0;
+    int cands[5] = {kBlockNRule};
+    int nc = 1;
     for (int bn : {256, 128, 64}) {
         if (N % bn != 0 || (epi == kEpiQuad && bn != 256) ||
             (epi == kEpiSubpel && (shape.sub_cout <= 0 || shape.sub_cout % bn != 0))) {
@@ -154,7 +186,7 @@ cudaError_t gemm_autotune(int dtype, int epi, const GemmParams& shape, cudaStrea
     if (gemm_stream_eligible(epi, M, N, K)) {
         cands[nc++] = kBlockNStream;  // the streaming form of the residual epilogues
     }
-    if (nc == 0) {
+    if (nc == 1) {
         return cudaErrorInvalidValue;
     }
     const size_t el = 2;  // f16 / bf16
@@ -199,7 +231,7 @@ cudaError_t gemm_autotune(int dtype, int epi, const GemmParams& shape, cudaStrea
         return e;
     }
     int best = 0;
-    float best_t = 0.f;
+    float best_t = 0.f, rule_t = 0.f;
     for (int i = 0; i < nc && e == cudaSuccess; ++i) {
         e = gemm_sm100(dtype, s.p[0], K, s.p[1], p, epi, cands[i], stream);  // warm-up
         if (e == cudaErrorInvalidValue) {
@@ -225,7 +257,9 @@ cudaError_t gemm_autotune(int dtype, int epi, const GemmParams& shape, cudaStrea
             e = cudaEventElapsedTime(&ms, ev[0], ev[1]);
         }
         const float us = ms * 1e3f / kTuneReps;
-        if (e == cudaSuccess && (best == 0 || us < best_t)) {
+        if (e == cudaSuccess && cands[i] == kBlockNRule) {
+            rule_t = us;
+        } else if (e == cudaSuccess && (best == 0 || us < best_t)) {
             best = cands[i];
             best_t = us;
         }
@@ -238,12 +272,7 @@ cudaError_t gemm_autotune(int dtype, int epi, const GemmParams& shape, cudaStrea
     if (best == 0) {
         return cudaErrorInvalidValue;
     }
-    {
-        std::lock_guard<std::mutex> lk(g_tune_mu);
-        g_tuned[TuneKey{current_device(), dtype, epi, M, N, K, epi == kEpiSubpel ? shape.sub_w : 0}] =
-            TuneEntry{best, best_t};
-        g_tuned_count.store(g_tuned.size(), std::memory_order_release);
-    }
+    record_tuned(dtype, epi, shape, TuneEntry{best, best_t, rule_t == 0.f || best_t < kTuneMargin * rule_t});
     if (best_bn != nullptr) {
         *best_bn = best;
     }
@@ -253,21 +282,22 @@ cudaError_t gemm_autotune(int dtype, int epi, const GemmParams& shape, cudaStrea
     return cudaSuccess;
 }
 
-// The codecs' hook: the tuned width of this shape, tuning it first when tuning is enabled, the
-// shape is new and the stream is not capturing; 0 (the library's rule) otherwise.
+// The codecs' hook: the width to use for this shape, 0 for the library's rule; tunes the shape first when tuning is
+// enabled, the shape is new and the stream is not capturing.  The quad epilogue has one width, so there is nothing
+// to measure (the rule picks its form).
 int gemm_bn_for(int dtype, int epi, const GemmParams& p, cudaStream_t stream)
 {
-    const int sub_w = epi == kEpiSubpel ? p.sub_w : 0;
-    const int bn = gemm_tuned_bn(dtype, epi, p.M, p.N, p.K, sub_w);
-    if (bn != 0 || !gemm_autotune_enabled()) {
-        return bn;
+    TuneEntry e{};
+    if (!find_tuned(dtype, epi, p.M, p.N, p.K, epi == kEpiSubpel ? p.sub_w : 0, &e) && gemm_autotune_enabled()) {
+        if (epi == kEpiQuad) {
+            record_tuned(dtype, epi, p, TuneEntry{256, 0.f, false});
+        } else if (gemm_autotune(dtype, epi, p, stream, nullptr, nullptr) != cudaSuccess) {
+            cudaGetLastError();  // an untunable shape keeps the library's rule
+            return 0;
+        }
+        return gemm_tuned_bn(dtype, epi, p.M, p.N, p.K, epi == kEpiSubpel ? p.sub_w : 0);
     }
-    int best = 0;
-    if (gemm_autotune(dtype, epi, p, stream, &best, nullptr) != cudaSuccess) {
-        cudaGetLastError();  // an untunable shape keeps the library's rule
-        return 0;
-    }
-    return best;
+    return e.beats_rule ? e.bn : 0;
 }
 
 }  // namespace dcvc

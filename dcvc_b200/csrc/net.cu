@@ -373,11 +373,10 @@ void gemm(Launch& L, const Lin& lin, int epi, const __half* x, int ldx, int M, _
     p.sub_cout = epi == kEpiSubpel ? lin.cout / 4 : 0;
     p.q_rows = q != nullptr ? q_rows : 0;
     p.err = L.err_word;
-    // the autotuned width of this shape (tuned here on first sight when tuning is enabled and
-    // the phase runs eagerly), else the library's rule
+    // the autotuned width of this shape where it beats the library's rule (tuned here on first sight when tuning
+    // is enabled and the phase runs eagerly)
     const int bn = gemm_bn_for(lin.dtype, epi, p, L.s);
-    // the quad epilogue has one width; the form stays the library's choice
-    L.note(gemm_sm100(lin.dtype, x, ldx, lin.w, p, epi, epi == kEpiQuad ? 0 : bn, L.s));
+    L.note(gemm_sm100(lin.dtype, x, ldx, lin.w, p, epi, bn, L.s));
 }
 
 void run_dcb(Launch& L, const Dcb& d, const __half* x, int ldx, int H, int W, __half* out, int ldo,

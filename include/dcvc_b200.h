@@ -129,12 +129,12 @@ int dcvc_quantize_fp8(const void* src, int src_dtype, int lds, float inv_scale, 
 /* Runtime autotuner of the dcvc_conv1x1 tile width.  Replaces the reference's compile-time
  * per-shape configuration tables (HINT_MAP_* in src/layers/extensions/inference/cutlass/
  * conv1x1_bias.cu:8 and its siblings, looked up by launch_cutlass_helper, cutlass_kernel.h:232-250).
- * dcvc_gemm_autotune times every valid N tile (256, 128, 64) of one shape (M, N, K, epilogue;
- * sub_w / sub_cout for SUBPEL) on zero-filled scratch operands on `stream`, which must not be
- * capturing, and records the fastest in a process-wide table; *block_n and *us (either may be
- * NULL) receive the choice and its time per launch.  dcvc_conv1x1 with block_n = 0 and the
- * codecs use a recorded width for their shape, else the library's rule.  The tile width changes
- * no output bit.  dcvc_gemm_autotune_enable(1) (or DCVC_GEMM_AUTOTUNE=1 in the environment) makes
+ * dcvc_gemm_autotune times the library's own choice and every valid N tile (256, 128, 64, and the
+ * streaming form where it exists) of one shape (M, N, K, epilogue; sub_w / sub_cout for SUBPEL) on
+ * zero-filled scratch operands on `stream`, which must not be capturing, and records the fastest tile in a
+ * process-wide table; *block_n and *us (either may be NULL) receive it and its time per launch.
+ * dcvc_conv1x1 with block_n = 0 and the codecs use a recorded tile for their shape if it was faster than
+ * the library's own choice, else that choice.  The form changes no output bit.  dcvc_gemm_autotune_enable(1) (or DCVC_GEMM_AUTOTUNE=1 in the environment) makes
  * the codecs tune every new shape on the first, eager run of a phase, before its graph is
  * captured.  dcvc_gemm_tuned reports the recorded width (0 = none); dcvc_gemm_tuning_clear
  * empties the table. */
