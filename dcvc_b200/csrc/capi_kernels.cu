@@ -76,9 +76,9 @@ int dcvc_gemm_stream_form(int enable)
     return kOk;
 }
 
-int dcvc_gemm_pair_form(int enable)
+int dcvc_gemm_pair_form(int form)
 {
-    gemm_set_pair_form(enable != 0);
+    gemm_set_pair_form(form);
     return kOk;
 }
 

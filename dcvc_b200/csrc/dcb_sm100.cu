@@ -729,7 +729,7 @@ bool dcb_tail_supported(int C, int cdc, int cffn, int n1)
 //     37888 19.3 / 19.3, 129600 58 / 58
 bool dcb_tail_preferred(int M, int C, int cdc, int cffn, int n1)
 {
-    if (!dcb_tail_supported(C, cdc, cffn, n1)) {
+    if (!gemm_pairs_allowed() || !dcb_tail_supported(C, cdc, cffn, n1)) {
         return false;
     }
     const int tiles = (M + 2 * kRows - 1) / (2 * kRows), pairs = num_sms() / 2;

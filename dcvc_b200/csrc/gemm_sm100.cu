@@ -793,10 +793,11 @@ int gemm_tuned_bn(int dtype, int epi, int M, int N, int K, int sub_w);
 namespace {
 std::atomic<int> g_stream_form{1};
 std::atomic<int> g_dw_fusion{0};
-std::atomic<int> g_pair_form{0};
+std::atomic<int> g_pair_form{-1};
 }  // namespace
 
-void gemm_set_pair_form(bool on) { g_pair_form.store(on ? 1 : 0); }
+void gemm_set_pair_form(int form) { g_pair_form.store(form < 0 ? -1 : (form > 0 ? 1 : 0)); }
+bool gemm_pairs_allowed() { return g_pair_form.load(std::memory_order_relaxed) != 0 && num_sms() >= 2; }
 
 void gemm_set_stream_form(int form) { g_stream_form.store(form < 0 ? 0 : (form > 2 ? 2 : form)); }
 bool gemm_stream_form_enabled() { return g_stream_form.load(std::memory_order_relaxed) != 0; }
@@ -806,7 +807,7 @@ bool gemm_dw_fusion_enabled() { return g_dw_fusion.load(std::memory_order_relaxe
 int gemm_pick_bn(int M, int N, int epi, int sub_cout, int K)
 {
     if (epi == kEpiQuad) {
-        if (N % 256 == 0 && g_pair_form.load(std::memory_order_relaxed) != 0 && num_sms() >= 2) {
+        if (N % 256 == 0 && g_pair_form.load(std::memory_order_relaxed) == 1 && num_sms() >= 2) {
             return kBlockNPair;
         }
         if (N % 256 != 0) {
@@ -889,7 +890,7 @@ static bool gemm_pair_preferred(int epi, int M, int N, int K)
 {
     const long long pairs = num_sms() / 2;
     const bool res = epi == kEpiBiasRes || epi == kEpiBiasResQ;
-    if ((epi != kEpiBias && epi != kEpiBiasWsilu && !res) || N % 256 != 0 || K < 512 || pairs < 1) {
+    if ((epi != kEpiBias && epi != kEpiBiasWsilu && !res) || N % 256 != 0 || K < 512 || !gemm_pairs_allowed()) {
         return false;
     }
     const long long cols = N / 256;

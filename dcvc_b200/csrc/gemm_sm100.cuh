@@ -104,8 +104,11 @@ bool gemm_stream_form_enabled();
 // Whether the codecs compute the depthwise 3x3 inside the streaming residual GEMM (default off:
 // measured slower than the two launches, see the kernel file).
 void gemm_set_dw_fusion(bool on);
-// Whether the library's own choice gives the quad GEMM the CTA-pair form (default off).
-void gemm_set_pair_form(bool on);
+// Whether the library's own choice may take kernels that work in CTA pairs (pair GEMM, resident quad, DepthConvBlock
+// tail): -1 where they are the faster ones (default), 0 never, 1 as -1 with every quad GEMM in the pair form; explicit
+// block_n values and dcvc_dcb_tail are not affected.
+void gemm_set_pair_form(int form);
+bool gemm_pairs_allowed();
 bool gemm_dw_fusion_enabled();
 // The quad epilogue with resident activations: K <= 512 16-bit values or 1024 bytes of E4M3 (a multiple
 // of 64, or 256), N a multiple of 256.  Bitwise the same outputs as gemm_sm100.

@@ -446,7 +446,7 @@ bool quad_sm100_eligible(int dtype, int M, int N, int K)
 // A unit takes a pair about as long as a tile takes one SM in the tiled kernel, so rounds are compared.
 bool quad_sm100_preferred(int dtype, int M, int N, int K)
 {
-    if (!quad_sm100_eligible(dtype, M, N, K)) {
+    if (!gemm_pairs_allowed() || !quad_sm100_eligible(dtype, M, N, K)) {
         return false;
     }
     const int sms = num_sms(), pairs = sms / 2;

@@ -103,14 +103,17 @@ int dcvc_conv1x1(int dtype, int epilogue, int M, int N, int K, const void* a, in
                  const void* w, const float* bias, const void* res, int ldr, const void* res2,
                  int ldr2, const void* qscale, void* out, int ldo, int sub_w, int sub_cout,
                  int block_n, void* stream);
-/* Which GEMMs the library's own tile choice (block_n = 0 without a tuned width, and the codecs)
- * gives the streaming form: 0 none, 1 the residual epilogues at K <= 256 (the default), 2 also
- * the bias and WSiLU epilogues at K <= 512.  Output bits are the same either way.  No counterpart
- * in the reference. */
+/* Which GEMMs the library's own choice (block_n = 0, and the codecs) gives the streaming form: 0 none, 1 the
+ * residual epilogues at K <= 256 where no narrower tile runs all at once (the default), 2 also the bias and
+ * WSiLU epilogues at K <= 512.  Output bits are the same either way.  No counterpart in the reference. */
 int dcvc_gemm_stream_form(int enable);
-/* Whether the library's own tile choice (and the codecs) gives the quad GEMM the CTA-pair form
- * (DCVC_BLOCK_N_PAIR): 1 or 0 (the default).  No counterpart in the reference. */
-int dcvc_gemm_pair_form(int enable);
+/* Whether the library's own choice (block_n = 0, dcvc_conv_ffn, and the codecs) takes the kernels that work in
+ * pairs of CTAs over two SMs: -1 where they are the faster ones (the default), 0 never (neither the pair form of the
+ * GEMM, nor the quad GEMM with resident activations, nor the DepthConvBlock tail in one kernel), 1 as -1 with every
+ * quad GEMM in the pair form (DCVC_BLOCK_N_PAIR).  With 0 and dcvc_gemm_stream_form(0) every GEMM is the tiled
+ * kernel of one CTA per tile.  Output bits are the same in every case.  A codec's recorded phases keep the forms
+ * they were recorded with.  No counterpart in the reference. */
+int dcvc_gemm_pair_form(int form);
 /* The FP8 form of dcvc_conv1x1 for the epilogues BIAS, BIAS_WSILU and QUAD: a [M, K] and
  * w [N, K] are E4M3 bytes (lda a multiple of 16, K of 128), the tcgen05 MMA is kind::f8f6f4
  * with FP32 accumulation, and the epilogue computes acc * wscale[n] + bias[n] (wscale: FP32
