@@ -20,6 +20,7 @@ import os
 import statistics
 import subprocess
 import sys
+import threading
 import time
 
 import numpy as np
@@ -45,7 +46,7 @@ WEIGHTS = ("seed-0 random init of the HT-S architecture (equal to the reference 
            "torch.manual_seed(0)), residual-branch output convs scaled x0.1 so activations stay "
            "finite in FP16 (the plain init grows ~1e14x per chunk, in FP64 too)")
 PUBLISHED = {"enc_fps_b200": 1415.1, "dec_fps_b200": 945.8, "combined_fps_derived": 567.0}
-QUAD_SHAPE = (32640, 1024, 512)  # ffn.0 of a 512-channel dcb2 DepthConvBlock at 1080p
+BLOCK_PIXELS = 32640  # rows of a DepthConvBlock of the 1/8 grid at 1080p (136 x 240)
 
 
 def parse_args():
@@ -127,7 +128,6 @@ class ClockSampler:
             cmd += ["-i", uuid]
         self.lines = []
         try:
-            import threading
             self.p = subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.DEVNULL, text=True)
             self.t = threading.Thread(target=self._read, daemon=True)
             self.t.start()
@@ -220,50 +220,47 @@ def _time_rotating(stream, launches, reps=60):
 
 
 def roofline(stream):
-    """The two largest kernels of the 1080p chunk, timed standalone on their launching stream
-    with CUDA events at their 1080p shapes and the library's own choice of kernel form:
-    the residual GEMM (dc.3 / ffn.2 of a 512-channel block, M=32640 N=512 K=256 + residual;
-    HBM-bound, the largest share of the chunk in the launch list) and the quad GEMM (ffn.0 +
-    WSiLU chunk-add, M=32640 N=1024 K=512; tensor-bound).  Operand sets rotate through more
-    than the 126 MB L2, so inputs come from HBM.  Returns (dominant, [others])."""
+    """The two largest kernels of the 1080p chunk, timed standalone on their launching stream with CUDA events at
+    their 1080p shapes and the library's own choice of kernel form: the tail of a 512-channel DepthConvBlock (dc.3 +
+    ffn.0 + ffn.2 in one kernel, M=32640) and its dc.0 (M=32640 N=256 K=512, WSiLU).  Operand sets rotate through
+    more than the 126 MB L2, so inputs come from HBM.  Returns (dominant, [others])."""
     from dcvc_b200 import _native as N, ops
     hbm, peak_tf, kind = measured_peaks()
     g = torch.Generator(device="cuda").manual_seed(7)
-    M = QUAD_SHAPE[0]
+    M = BLOCK_PIXELS
 
     def rnd(*shape, scale=1.0):
         return (torch.randn(*shape, device="cuda", generator=g) * scale).half()
 
-    # residual GEMM: three operand sets of 83.5 MB
-    res_launch = []
+    # the tail: three operand sets of 83.6 MB (operand, residual, output) and the 1.6 MB of weights
+    tail_launch = []
     for _ in range(3):
-        a, w = rnd(M, 256), rnd(512, 256, scale=256 ** -0.5)
-        r, o = rnd(M, 512), torch.empty(M, 512, device="cuda", dtype=torch.float16)
-        b = torch.zeros(512, device="cuda")
-        res_launch.append(lambda a=a, w=w, b=b, r=r, o=o: ops.conv1x1(a, w, b, N.EPI_BIAS_RES, res=r, out=o))
-    sec = _time_rotating(stream, res_launch)
-    byts = (M * 256 + 512 * 256 + 2 * M * 512) * 2
-    res = {"kernel": "gemm_stream_kernel<half, res> (dc.3 / ffn.2 + bias + residual, M=32640 N=512 "
-                     "K=256; the streaming form the library picks for these shapes)",
-           "bound": "hbm", "achieved": round(byts / sec / 1e9, 1), "peak": hbm, "unit": "GB/s",
-           "frac": round(byts / sec / 1e9 / hbm, 3), "peak_kind": f"{kind} HBM copy",
-           "us_per_launch": round(sec * 1e6, 2), "bytes_per_launch": byts,
-           "traffic": profiled_traffic("gemm_res_stream_1080p")}
-    # quad GEMM: three operand sets (A 33.4 MB + out 16.7 MB each, plus the 1 MB weights)
-    quad_launch = []
-    for _ in range(3):
-        a, w = rnd(M, 512), rnd(1024, 512, scale=512 ** -0.5)
-        o = torch.empty(M, 256, device="cuda", dtype=torch.float16)
-        b = torch.zeros(1024, device="cuda")
-        quad_launch.append(lambda a=a, w=w, b=b, o=o: ops.conv1x1(a, w, b, N.EPI_QUAD, out=o))
-    sec = _time_rotating(stream, quad_launch)
-    flops = 2.0 * M * 1024 * 512
-    quad = {"kernel": "gemm_sm100_kernel<half, 256, quad> (ffn.0 + WSiLU chunk-add, M=32640 N=1024 K=512)",
+        a, x, o = rnd(M, 256), rnd(M, 512), torch.empty(M, 512, device="cuda", dtype=torch.float16)
+        w = (rnd(512, 256, scale=256 ** -0.5), torch.zeros(512, device="cuda"), rnd(1024, 512, scale=512 ** -0.5),
+             torch.zeros(1024, device="cuda"), rnd(512, 256, scale=256 ** -0.5), torch.zeros(512, device="cuda"))
+        tail_launch.append(lambda a=a, x=x, w=w, o=o: ops.dcb_tail(a, x, *w, out=o))
+    sec = _time_rotating(stream, tail_launch)
+    flops = 2.0 * M * (512 * 256 + 1024 * 512 + 512 * 256)
+    tail = {"kernel": "dcb_tail_kernel<half, 512, 256, 256> (dc.3 + residual, ffn.0 + WSiLU chunk-add, ffn.2 + "
+                      "residual, M=32640)",
             "bound": "tensor", "achieved": round(flops / sec / 1e12, 1), "peak": peak_tf,
             "unit": "TFLOP/s", "frac": round(flops / sec / 1e12 / peak_tf, 3),
             "peak_kind": f"{kind} bf16 burst", "us_per_launch": round(sec * 1e6, 2),
-            "flops_per_launch": flops, "traffic": profiled_traffic("gemm_quad_1080p")}
-    return res, [quad]
+            "flops_per_launch": flops, "traffic": profiled_traffic("dcb_tail_1080p")}
+    # dc.0: four operand sets of 50.1 MB
+    dc0_launch = []
+    for _ in range(4):
+        a, w = rnd(M, 512), rnd(256, 512, scale=512 ** -0.5)
+        o, b = torch.empty(M, 256, device="cuda", dtype=torch.float16), torch.zeros(256, device="cuda")
+        dc0_launch.append(lambda a=a, w=w, b=b, o=o: ops.conv1x1(a, w, b, N.EPI_BIAS_WSILU, out=o))
+    sec = _time_rotating(stream, dc0_launch)
+    byts = (M * 512 + 256 * 512 + M * 256) * 2 + 256 * 4
+    dc0 = {"kernel": "gemm_sm100_kernel<half, 256, bias + WSiLU, CTA pairs> (dc.0, M=32640 N=256 K=512)",
+           "bound": "hbm", "achieved": round(byts / sec / 1e9, 1), "peak": hbm, "unit": "GB/s",
+           "frac": round(byts / sec / 1e9 / hbm, 3), "peak_kind": f"{kind} HBM copy",
+           "us_per_launch": round(sec * 1e6, 2), "bytes_per_launch": byts,
+           "traffic": profiled_traffic("gemm_pair_wsilu_1080p")}
+    return tail, [dc0]
 
 
 class ReferenceCpuPath:
@@ -466,7 +463,6 @@ def batched_form(args):
     Plain: the same chunks coded one request at a time by single-stream FP16 codecs (the
     reference's form).  Both encode and decode every chunk; both are device-timed from one start
     event to one end event.  Reported in frames/s and 1080p-equivalent frames/s (pixels)."""
-    import threading
     from dcvc_b200 import synthetic
     from dcvc_b200.entropy_tables import add_cdf_to_state_dict
     from dcvc_b200.inference_extensions_cuda import DMCHTSProxy
@@ -911,6 +907,54 @@ def _section(fn, *a):
         return {"error": f"{type(e).__name__}: {e}"[:300]}
 
 
+class Deadlines:
+    """The output line and a limit on the host for each part of the run.  A call that never returns (a launch that
+    does not end, a request that is never answered) cannot be interrupted from Python, so when a part outlives its
+    limit a watcher thread writes that into the part's key, prints the line with everything measured before it and
+    ends the process; before the headline value is known there is no line and the process fails."""
+
+    def __init__(self, out, prints=True):
+        self.out = out
+        self.prints = prints
+        self.ready = False  # the line has its headline value
+        self._lock = threading.Lock()
+        self._part = None   # (key, seconds, end)
+        threading.Thread(target=self._watch, daemon=True).start()
+
+    def run(self, key, seconds, fn, *a):
+        """out[key] = _section(fn, *a) within `seconds`."""
+        with self._lock:
+            self._part = (key, seconds, time.monotonic() + seconds)
+        value = _section(fn, *a)
+        with self._lock:
+            self._part = None
+            self.out[key] = value
+        return value
+
+    def start(self, key, seconds):
+        with self._lock:
+            self._part = (key, seconds, time.monotonic() + seconds)
+
+    def stop(self):
+        with self._lock:
+            self._part = None
+
+    def _watch(self):
+        while True:
+            time.sleep(0.2)
+            with self._lock:
+                if self._part is None or time.monotonic() < self._part[2]:
+                    continue
+                key, seconds, _ = self._part
+                if not self.ready:
+                    print(f"bench: {key} did not end within {seconds} s", file=sys.stderr, flush=True)
+                    os._exit(1)
+                self.out[key] = {"error": f"did not end within {seconds} s; the parts after it were not run"}
+                if self.prints:
+                    print(json.dumps(self.out), flush=True)
+                os._exit(0)
+
+
 def _empty_cache():
     try:
         torch.cuda.empty_cache()
@@ -926,7 +970,12 @@ def run_reference(args):
     if rank != 0:
         return
     H, W = args.height, args.width
-    path = ReferenceCpuPath(H, W)
+    try:
+        path = ReferenceCpuPath(H, W)
+    except FileNotFoundError as e:
+        print(json.dumps({"impl": "reference", "unavailable": "the reference's rANS coder, compiled from its sources, "
+                          f"is not there: {os.path.relpath(str(e), ROOT)}"}), flush=True)
+        return
     for i in range(args.warmup):
         path.chunk(i)
     per_step = []
@@ -967,6 +1016,9 @@ def run_gpu(args):
     from dcvc_b200.model_spec import calibrated_hts_state_dict
 
     H, W = args.height, args.width
+    out = {}
+    parts = Deadlines(out, prints=rank == 0)
+    parts.start("the headline measurement", 400)
     sd = add_cdf_to_state_dict(calibrated_hts_state_dict(0))
     sd = {k: (v.half().cuda() if v.is_floating_point() else v) for k, v in sd.items()}
     stream = torch.cuda.Stream()
@@ -1072,38 +1124,8 @@ def run_gpu(args):
     windows[-1][1] = time.time()
     e2e = FRAMES * args.steps * world / (max_over_ranks(e0.elapsed_time(e1), "cuda") / 1e3)
 
-    # ---------------- encode alone and decode alone (the reference publishes them separately)
-    split = split_enc_dec(enc, dec, xs, args, pb, pr, H, W, stream)
-    # ---------------- the same workload in the BF16 and FP8 precision forms
-    forms = _section(precision_forms, stream, H, W, xs, args.steps, args.warmup)
-    clk = clocks.stop(windows)
-    roof, roof_others = roofline(stream)
-    # The extra measurements below report a failure in their own key instead of losing the line
-    # (and every rank still reaches the closing barrier).
-    intra = None if args.no_intra else _section(intra_bench, stream, H, W)
-    htl = None if args.no_htl else _section(htl_bench, stream, H, W)
-    ld = None if args.no_ld else _section(ld_bench, stream, H, W)
-    del enc, dec
-    _empty_cache()
-    batched = _section(batched_form, args) if args.batch_streams > 0 else None
-    _empty_cache()
-    # a one-GPU measurement: under torchrun the ranks skip it
-    serving = None
-    if args.serve_seconds > 0 and world == 1:
-        serving = _section(serving_bench, args)
-    _empty_cache()
-    cpu = None
-    parity = None
-    if rank == 0 and world == 1 and not args.no_cpu_baseline:
-        cpu = cpu_baseline(H, W)
-        parity = _section(parity_vs_fp64_oracle, H, W)
-    if world > 1:
-        dist.barrier()
-        dist.destroy_process_group()
-    if rank != 0:
-        return
     lat_sorted = sorted(lat)
-    out = {
+    out.update({
         "metric": METRIC, "value": round(value, 2), "unit": UNIT, "n_gpus": world,
         "steps": args.steps, "warmup": args.warmup, "ms_per_step": round(ms_max / args.steps, 3),
         "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f16",
@@ -1111,25 +1133,51 @@ def run_gpu(args):
         "latency_ms": {"p50": round(float(np.percentile(lat_sorted, 50)), 3),
                        "p99": round(float(np.percentile(lat_sorted, 99)), 3)},
         "bytes_per_chunk": {"mean": int(np.mean(nbytes)), "min": int(min(nbytes)), "max": int(max(nbytes))},
-        "enc_decomposed_fps": split,
-        "precision_forms": forms,
-        "batched": batched,
-        "serving": serving,
         "reference_published": PUBLISHED,
-        "intra": intra,
-        "htl": htl,
-        "ld": ld,
         "e2e": {"value": round(e2e, 2), "unit": UNIT, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                 "io": "8-bit YUV 4:2:0 planes in and out, converted on the device; copies on a second "
                       "stream, double-buffered, inside the timed region"},
         "gpu_launches": kernels_per_step * args.steps,
-        "roofline": roof,
-        "roofline_others": roof_others,
-        "clocks": clk,
-        "cpu_baseline": cpu,
-        "parity": parity,
-    }
-    print(json.dumps(out), flush=True)
+        "clocks": clocks.stop(windows),
+        "enc_decomposed_fps": None, "precision_forms": None, "roofline": None, "roofline_others": None,
+        "intra": None, "htl": None, "ld": None, "batched": None, "serving": None, "cpu_baseline": None,
+        "parity": None,
+    })
+    parts.ready = True
+    # The parts below report a failure, or that they did not end, in their own key instead of losing the line
+    # (and every rank still reaches the closing barrier).  Limits: several times what each takes.
+    # ---------------- encode alone and decode alone (the reference publishes them separately)
+    parts.run("enc_decomposed_fps", 60, split_enc_dec, enc, dec, xs, args, pb, pr, H, W, stream)
+    # ---------------- the same workload in the BF16 and FP8 precision forms
+    parts.run("precision_forms", 120, precision_forms, stream, H, W, xs, args.steps, args.warmup)
+    roof = parts.run("roofline", 60, roofline, stream)
+    if isinstance(roof, tuple):
+        out["roofline"], out["roofline_others"] = roof
+    if not args.no_intra:
+        parts.run("intra", 90, intra_bench, stream, H, W)
+    if not args.no_htl:
+        parts.run("htl", 90, htl_bench, stream, H, W)
+    if not args.no_ld:
+        parts.run("ld", 90, ld_bench, stream, H, W)
+    del enc, dec
+    _empty_cache()
+    if args.batch_streams > 0:
+        parts.run("batched", 240, batched_form, args)
+    _empty_cache()
+    # a one-GPU measurement: under torchrun the ranks skip it
+    if args.serve_seconds > 0 and world == 1:
+        parts.run("serving", 240, serving_bench, args)
+    _empty_cache()
+    if rank == 0 and world == 1 and not args.no_cpu_baseline:
+        parts.run("cpu_baseline", 240, cpu_baseline, H, W)
+        parts.run("parity", 420, parity_vs_fp64_oracle, H, W)
+    if world > 1:
+        parts.start("closing_barrier", 300)
+        dist.barrier()
+        dist.destroy_process_group()
+    parts.stop()
+    if rank == 0:
+        print(json.dumps(out), flush=True)
 
 
 def main():
