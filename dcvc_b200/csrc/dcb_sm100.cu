@@ -719,14 +719,16 @@ bool dcb_tail_supported(int C, int cdc, int cffn, int n1)
 // The kernel's time goes in waves of one tile per pair of SMs, that of the separate launches with M, by a
 // step where the 256 columns of dc.3 and ffn.2 (128-wide tiles of 512) no longer run in one round, at
 // 128 * num_sms / 4 rows (one B200, inputs rotating through L2, microseconds fused / separate):
-//   (512, 256, 256): M = 4736 21.5 / 16.9, 5120 21.5 / 22.5, 14400 23.7 / 35.7, 22528 (second wave a
-//     fifth full) 45.5 / 44.8, 25600 46.2 / 50.3, 32640 48.3 / 59.2, 129600 173 / 215
-//   (256, 256, 256): M = 4736 14.7 / 13.7, 5120 14.7 / 16.4, 14400 16.1 / 26.8, 19200 27.0 / 31.9
-//   (256, 128, 128): M = 2304 11.2 / 9.3, 4736 11.3 / 11.4, 5120 11.3 / 13.7, 14400 12.5 / 20.2, 19200
-//     20.1 / 24.9, 129600 69 / 88
+//   (512, 256, 256): M = 4736 22.1 / 16.9, 6144 22.5 / 23.5, 14400 24.3 / 36.2; 19200 (second wave just begun) 45.8 /
+//     43.3, 23552 (a quarter full) 49.9 / 48.5, 24576 50.7 / 53.0, 32640 51.3 / 60.8; 38400 (third wave) 77.8 / 75.6,
+//     42000 (almost a quarter) 80.0 / 77.6, 44000 77.5 / 81.7; 57600 (fourth) 108.7 / 107.5; 129600 202 / 226
+//   (256, 256, 256): M = 4736 20.0 / 18.3, 5120 15.3 / 16.4, 14400 18.4 / 29.0, 19200 27.7 / 32.7, 38400 44.1 / 46.7,
+//     129600 107 / 135
+//   (256, 128, 128): M = 4736 13.1 / 12.3, 5120 12.5 / 14.4, 14400 13.8 / 21.3, 19200 21.0 / 26.1, 38400 32.5 / 36.5,
+//     129600 71 / 91
 // and against the one-SM ConvFFN kernel (ffn_sm100.cu; cdc = 0):
-//   (512, 256): M = 390 17.4 / 38.6, 32640 39.5 / 90.9;  (256, 128): M = 390 9.2 / 11.6, 14400 10.3 / 12.6,
-//     37888 19.3 / 19.3, 129600 58 / 58
+//   (512, 256): M = 390 17.1 / 38.6, 32640 40.0 / 89.0;  (256, 128): M = 390 9.2 / 11.6, 14400 10.9 / 13.3,
+//     37888 18.6 / 19.2, 48000 27.2 / 26.7, 129600 57.7 / 59.4
 bool dcb_tail_preferred(int M, int C, int cdc, int cffn, int n1)
 {
     if (!gemm_pairs_allowed() || !dcb_tail_supported(C, cdc, cffn, n1)) {
@@ -736,7 +738,8 @@ bool dcb_tail_preferred(int M, int C, int cdc, int cffn, int n1)
     if (cdc == 0) {
         return cffn == 256 || tiles <= 2 * pairs;
     }
-    if (C == 512 && tiles > pairs && 8 * tiles < 10 * pairs) {
+    const int over = tiles % pairs;  // tiles of a last wave that is not full
+    if (C == 512 && over > 0 && 4 * over < pairs && (tiles / pairs == 1 || tiles / pairs == 2)) {
         return false;
     }
     return 4LL * ((M + kRows - 1) / kRows) > num_sms();

@@ -880,24 +880,24 @@ GemmParams gemm_apply_injection(const GemmParams& p)
 
 // Whether CTA pairs (256 x 256 tiles, each CTA staging half of the W tile) beat one CTA per 128 x 256 tile
 // where no narrower tile runs all at once.  A K block of a pair stages 32 KB per CTA instead of 48 KB, which pays
-// once the K loop is long enough to wait on its copies: from K = 512 (us back to back, one CTA / pair: WSiLU
-// 14400 x 512 x 512 12.6 / 11.6, 14400 x 768 x 768 20.7 / 18.0, 32640 x 512 x 512 21.2 / 19.2, residual 14400 x
-// 512 x 512 15.7 / 14.4, 32640 x 512 x 512 27.7 / 22.7, 32640 x 768 x 768 56.2 / 44.8; at K = 256 WSiLU 32640 x
-// 256 10.2 / 10.4).  The larger tile must not need a round more (6240 x 768 x 768 10.0 / 12.5), and where one
-// CTA per tile runs in one round only the residual epilogues gain, whose pairs have more stages beside the
-// residual (8160 x 512 x 512 WSiLU 8.7 / 9.0, residual 10.4 / 10.1).
+// once the K loop is long enough to wait on its copies: from K = 512 (us back to back, medians of alternating runs,
+// one CTA / pair: WSiLU 14400 x 768 x 768 21.6 / 18.5, 32640 x 512 x 512 22.1 / 20.3, residual 14400 x 512 x 512 14.6 /
+// 13.4, 32640 x 512 x 512 28.0 / 24.1, 32640 x 768 x 768 57.2 / 46.5, bias 14400 x 512 x 2048 34.8 / 29.9; at K = 256
+// WSiLU 32640 x 256 10.2 / 10.4).  The larger tile must not need a round more (6240 x 768 x 768 10.0 / 12.5), and where
+// one CTA per tile runs in one round the pair's start costs more than its stages save (8160 x 512 x 512 WSiLU 8.7 /
+// 9.0, residual 8.2 / 9.1, 4736 x 768 x 768 residual 10.3 / 11.6).
 static bool gemm_pair_preferred(int epi, int M, int N, int K)
 {
     const long long pairs = num_sms() / 2;
-    const bool res = epi == kEpiBiasRes || epi == kEpiBiasResQ;
-    if ((epi != kEpiBias && epi != kEpiBiasWsilu && !res) || N % 256 != 0 || K < 512 || !gemm_pairs_allowed()) {
+    if ((epi != kEpiBias && epi != kEpiBiasWsilu && epi != kEpiBiasRes && epi != kEpiBiasResQ) || N % 256 != 0 || K < 512 ||
+        !gemm_pairs_allowed()) {
         return false;
     }
     const long long cols = N / 256;
     const long long tiles = (static_cast<long long>(M) + kBM - 1) / kBM * cols;
     const long long ptiles = (static_cast<long long>(M) + 2 * kBM - 1) / (2 * kBM) * cols;
     const long long rounds = (tiles + num_sms() - 1) / num_sms();
-    return (res || rounds > 1) && (ptiles + pairs - 1) / pairs <= rounds;
+    return rounds > 1 && (ptiles + pairs - 1) / pairs <= rounds;
 }
 
 // Host launcher.  A: [M, K] with row pitch lda (elements); W: [N, K] dense.  dtype 0 = f16,

@@ -435,15 +435,18 @@ bool quad_sm100_eligible(int dtype, int M, int N, int K)
            static_cast<long long>((M + 2 * kRows - 1) / (2 * kRows)) * (N / kNB) < 0x7fffffff;
 }
 
-// Whether it is the faster form where no narrower tile runs all at once (gemm_pick_bn; us back to back, tiled / this; M x N x K):
-//   16-bit: 390 x 1024 x 512 6.8 / 6.6, 1560 x 2048 x 512 (56 units on 74 pairs) 7.4 / 7.9,
-//   6240 x 1024 x 512 10.7 / 10.6, 8160 x 2048 x 512 18.3 / 16.9, 32640 x 1024 x 512 30.2 / 28.0, 32640 x
-//   1536 x 384 54.5 / 32.5, 129600 x 1024 x 512 138 / 98
-//   E4M3: 390 x 1024 x 512 6.1 / 5.9, 6240 x 1024 x 512 8.9 / 9.4, 14400 x 1024 x 512 15.1 / 13.3, 32640 24.0 /
-//   20.5, 129600 76.9 / 66.0
-//   and where the last round of units is nearly empty: 6240 x 1536 x 384 (150 units) 9.8 / 11.2, 3600 x 2048
-//   x 512 (120) 10.0 / 10.6
-// A unit takes a pair about as long as a tile takes one SM in the tiled kernel, so rounds are compared.
+// Whether it is the faster form where no narrower tile runs all at once (gemm_pick_bn; us back to back, medians of
+// alternating runs, tiled / this; M x N x K):
+//   16-bit: 8160 x 1024 x 512 (128 units on 74 pairs) 9.7 / 11.0, 14400 (228) 15.4 / 15.8, 24000 (376) 23.6 / 24.0,
+//   32640 (512) 33.5 / 30.2, 129600 134 / 103; 14400 x 1536 x 384 (342) 17.4 / 17.7, 24000 (564) 27.2 / 27.3, 32640
+//   (768) 37.6 / 32.5; 12000 x 2048 x 512 (376) 23.7 / 24.4, 14400 (456) 27.6 / 26.9; 24000 x 1024 x 256 (376) 15.6 /
+//   16.0, 32640 (512) 18.5 / 18.1; 32640 x 512 x 256 (256) 11.9 / 12.6
+//   E4M3: 390 x 1024 x 512 5.7 / 6.0, 2040 5.9 / 6.2, 10000 (160) 11.3 / 11.0, 14400 (228) 13.9 / 13.0, 32640 22.4 /
+//   19.7
+// The tiled kernel's CTAs start on their own and it has stages for its first K blocks at once; the pair meets its
+// peer, fills both CTAs' slabs and then runs the units of its range without a gap, so it needs some of them: six per
+// pair, two of the shorter E4M3 ones.  A unit takes a pair about as long as a tile takes one SM in the tiled
+// kernel, so rounds are compared.
 bool quad_sm100_preferred(int dtype, int M, int N, int K)
 {
     if (!gemm_pairs_allowed() || !quad_sm100_eligible(dtype, M, N, K)) {
@@ -452,10 +455,7 @@ bool quad_sm100_preferred(int dtype, int M, int N, int K)
     const int sms = num_sms(), pairs = sms / 2;
     const long long blocks = N / kNB;
     const long long units = (M + 2 * kRows - 1) / (2 * kRows) * blocks, tiles = (M + kRows - 1) / kRows * blocks;
-    if (dtype == kDtypeF8 && 2 * units <= pairs) {
-        return true;
-    }
-    return 10 * units >= (dtype == kDtypeF8 ? 20 : 17) * pairs && (units + pairs - 1) / pairs <= (tiles + sms - 1) / sms;
+    return units >= (dtype == kDtypeF8 ? 2 : 6) * pairs && (units + pairs - 1) / pairs <= (tiles + sms - 1) / sms;
 }
 
 cudaError_t quad_sm100(int dtype, const void* A, int lda, const void* W, const GemmParams& p, cudaStream_t stream)
