@@ -1,7 +1,7 @@
 """Micro-benchmark of the codec's kernels at their 1080p shapes (CUDA events on the launching
 stream), also the small fixed case used for ncu captures.
 
-    python -m dcvc_b200.kernel_bench [--case quad|quad_f8|wsilu|res|dwres|dwres_split|bias2048|dwconv|ffn|ffn_ld|unshuffle|shuffle|quantize|rans|all]
+    python -m dcvc_b200.kernel_bench [--case tail|quad|quad_f8|wsilu|res|dwres|dwres_split|bias2048|dwconv|ffn|ffn_ld|unshuffle|shuffle|quantize|rans|all]
                                      [--reps N] [--sets S] [--bn 0|64|128|256|-1]
 
 (--bn -1 selects the streaming form of the residual GEMM.)
@@ -12,7 +12,8 @@ inside a chunk.
 
 Shapes are those of a 512-channel dcb2 DepthConvBlock at 1920x1088 (M = 136 x 240 = 32640
 pixels): dc.0 (512 -> 256, WSiLU), depthwise 3x3 on 256 channels, dc.3 (256 -> 512 + residual),
-ffn.0 (512 -> 4 x 256, WSiLU chunk-add), and the encoder's 2048 -> 512 adaptor.  `dwres` is the
+ffn.0 (512 -> 4 x 256, WSiLU chunk-add), and the encoder's 2048 -> 512 adaptor.  `tail` is dc.3, ffn.0 and
+ffn.2 (256 -> 512 + residual) in one kernel, as the codecs run them at this size.  `dwres` is the
 depthwise 3x3 and dc.3 in one launch (the depthwise form of the streaming residual GEMM),
 `dwres_split` the same two steps as two launches.
 """
@@ -31,6 +32,13 @@ def _case(name, g, bn=0):
     def rnd(*s, scale=1.0):
         return (torch.randn(*s, device="cuda", generator=g) * scale).half()
 
+    if name == "tail":
+        a, x, out = rnd(M8, 256), rnd(M8, 512), torch.empty(M8, 512, device="cuda", dtype=torch.float16)
+        w0, w1, w2 = rnd(512, 256, scale=1 / 16), rnd(1024, 512, scale=512 ** -0.5), rnd(512, 256, scale=1 / 16)
+        b = torch.zeros(1024, device="cuda")
+        fn = lambda: ops.dcb_tail(a, x, w0, b, w1, b, w2, b, out=out)  # noqa: E731
+        return fn, 2.0 * M8 * 5 * 512 * 256 + 2.0 * M8 * 512 * 256, \
+            (a.numel() + 2 * x.numel() + w0.numel() + w1.numel() + w2.numel()) * 2
     if name in ("ffn", "ffn_ld"):
         # the fused ConvFFN (quad GEMM + residual GEMM in one kernel) of a 512-channel dcb2 block
         # ("ffn") or of a 256-channel one, the LD codec's ("ffn_ld")
@@ -232,7 +240,7 @@ def main():
     ap.add_argument("--bn", type=int, default=0,
                     help="GEMM N tile (0 = the library's choice, -1 = streaming residual form)")
     args = ap.parse_args()
-    cases = ["quad", "wsilu", "res", "bias2048", "dwconv", "ffn"] if args.case == "all" else [args.case]
+    cases = ["tail", "quad", "wsilu", "res", "bias2048", "dwconv", "ffn"] if args.case == "all" else [args.case]
     for c in cases:
         if c == "rans":
             print(json.dumps(rans()), flush=True)
