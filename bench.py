@@ -271,15 +271,24 @@ class ReferenceCpuPath:
     (oracle/_ref), or, where that module is absent, taken from the reference's own tables
     committed as a fixture (tests/golden/cdf_tables.npz); nothing here loads libdcvc_b200.so.
 
+    `own_coder`: where the reference's coder is not built, the oracle's C restatement of it (same bytes) instead of
+    an error; the reference arm never asks for that.
+
     One chunk = the full H x W 8-frame chunk compressed by one instance and decompressed by a
     second one, QP cycling as in the GPU arm."""
 
-    def __init__(self, H, W, threads=None):
+    def __init__(self, H, W, threads=None, own_coder=False):
         sys.path.insert(0, os.path.join(ROOT, "oracle"))
         import hts_oracle
         from dcvc_b200 import synthetic
         from dcvc_b200.model_spec import calibrated_hts_state_dict
-        hts_oracle.use_reference_coder(True)
+        self.coder = "reference rANS coder compiled from the reference sources"
+        try:
+            hts_oracle.use_reference_coder(True)
+        except FileNotFoundError:
+            if not own_coder:
+                raise
+            self.coder = "the oracle's C restatement of the reference's rANS coder (the reference's is not built here)"
         self.threads = threads or os.cpu_count() or 1
         torch.set_num_threads(self.threads)
         sd = calibrated_hts_state_dict(0)
@@ -295,7 +304,6 @@ class ReferenceCpuPath:
         self.pr, self.pb = synthetic.padding_for(H, W)
         self.xs = [synthetic.to_model_input(synthetic.video_chunk_yuv420(2, H, W, FRAMES, FRAMES * k),
                                             device="cpu") for k in range(2)]
-        self.coder = "reference rANS coder compiled from the reference sources"
 
     def chunk(self, i):
         qp = QPS[i % len(QPS)]
@@ -336,7 +344,7 @@ def _reference_cdf_tables(sd):
 def cpu_baseline(H, W, chunks=2):
     """The reference's CPU path (ReferenceCpuPath) on all host cores, timed over `chunks` whole
     H x W chunks after one untimed chunk (a bounded sample of the workload, not scaled)."""
-    path = ReferenceCpuPath(H, W)
+    path = ReferenceCpuPath(H, W, own_coder=True)
     path.chunk(0)
     t0 = time.perf_counter()
     for k in range(chunks):

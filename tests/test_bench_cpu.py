@@ -51,3 +51,11 @@ def test_reference_arm_says_why_it_cannot_run():
     assert r.returncode == 0, r.stderr
     line = json.loads(r.stdout)
     assert line["impl"] == "reference" and "librans_ref.so" in line["unavailable"]
+
+
+def test_cpu_baseline_runs_without_the_references_coder():
+    r = subprocess.run([sys.executable, "-c", "import json, bench; print(json.dumps(bench.cpu_baseline(128, 128, 1)))"],
+                       cwd=ROOT, capture_output=True, text=True, timeout=200)
+    assert r.returncode == 0, r.stderr
+    out = json.loads(r.stdout)
+    assert out["value"] > 0 and "rANS coder" in out["sample"]
