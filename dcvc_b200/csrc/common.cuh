@@ -480,14 +480,18 @@ __device__ __forceinline__ void tma_load_2d_pair(void* dst, const void* tmap, ui
         : "memory");
 }
 
+// A CTA that holds tensor memory asks for more than half of an SM's shared memory, so that no two of them meet on one
+// SM and an allocation never waits for a kernel that waits for something else.
+constexpr int kTmemCtaMinSmem = 232448 / 2 + 1;
+
 // Tensor memory of a CTA pair.  tcgen05.alloc and tcgen05.dealloc with cta_group::2 are made by a warp of each
 // CTA together and act on the tensor memory of both SMs.  Nothing but a barrier of the cluster shows that the
-// other CTA has started, or that it is still there: a CTA that asks for the pair's columns before its peer
-// runs, or leaves while the peer still gives its columns back, has no bound on when (or whether) that operation
-// ends.  With one stream the two CTAs of a cluster start and end within some hundred clocks of each other; with
-// several codecs on the GPU one SM of a pair can be long in reaching the CTA.  Hence pair_begin() and pair_end().
+// other CTA has started, or that it is still there: without one, a CTA that asks for the pair's columns before its
+// peer runs, or leaves while the peer still gives its columns back, has no bound on when that operation ends.
+// Hence pair_begin() and pair_end(); the two meetings cost a launch 0.2 to 0.4 us (tail of 8160 to 14400 rows).
 
-// All threads of both CTAs, once the barriers of the CTA are initialised: the warp of each CTA for which `alloc_warp` holds allocates.
+// All threads of both CTAs, once the barriers of the CTA are initialised; the warp of each CTA for which `alloc_warp`
+// holds allocates.
 __device__ __forceinline__ uint32_t pair_begin(uint32_t* dst_smem, uint32_t ncols, bool alloc_warp)
 {
     cluster_sync();  // both CTAs run; their barriers are initialised before any copy or arrive reaches them

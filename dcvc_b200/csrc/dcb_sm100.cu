@@ -103,6 +103,7 @@ struct TailCfg {
     static_assert(kAccCol >= F / 2 && kAccCol + kAccs * kNB <= kTmemCols, "tensor memory");
     static_assert(K0 == 0 || kOwnA || 2 * K0 <= C, "dc.3 operand in the upper half of x");
     static_assert(kStages >= 3 && kBytes <= kSmemLimit && kBars * 8 + 8 <= kBarBytes, "shared memory");
+    static_assert(kBytes >= kTmemCtaMinSmem, "one CTA per SM");
     // ffn.2's blocks in the order that frees the dc.3 operand's slabs first
     static __device__ __forceinline__ int out_block(int i)
     {

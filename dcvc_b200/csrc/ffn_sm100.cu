@@ -50,6 +50,7 @@ struct FfnCfg {
     static constexpr int kTmemCols = 2 * BN;               // two accumulators
     static_assert(kStages >= 2, "shared memory too small for two pipeline stages");
     static_assert(kBytes <= kSmemLimit, "shared memory budget exceeded");
+    static_assert(kBytes >= kTmemCtaMinSmem, "one CTA per SM");
 };
 
 // Byte offset of 16-byte chunk j of row r in a 128-byte-swizzled tile (the layout TMA writes for

@@ -109,6 +109,7 @@ struct GemmCfg {
     static constexpr int kTmemCols = 2 * BN;
     static_assert(kStages >= 2, "shared memory too small for two pipeline stages");
     static_assert(kBytes <= kSmemLimit, "shared memory budget exceeded");
+    static_assert(kBytes >= kTmemCtaMinSmem, "one CTA per SM");
     static_assert(kDirect || kBoxes * kAccPerBox == kCols, "box tiling");
     static_assert(kDirect || kOutW * 2 == 128 || kOutW * 2 == 64, "staging row width");
     static_assert(kEpiWarps <= kMaxEpiWarps, "epilogue warps");

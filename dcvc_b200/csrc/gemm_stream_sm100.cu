@@ -100,6 +100,7 @@ struct StreamCfg {
     static constexpr int kBiasBytes = DW ? kSEpiWarps * kSCols * 4 : 0;
     static constexpr int kBytes = kBiasOffset + kBiasBytes + 1024;
     static_assert(kBytes <= 232448, "shared memory budget exceeded");
+    static_assert(kBytes >= kTmemCtaMinSmem, "one CTA per SM");
     static_assert(kEpiOffset % 1024 == 0 && kHaloOffset % 1024 == 0, "TMA destinations stay aligned");
 };
 

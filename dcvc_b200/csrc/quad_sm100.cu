@@ -86,6 +86,7 @@ __host__ __device__ inline QuadLayout quad_layout(int kslabs, int n)
     l.bias_offset = l.slabs * kSlabBytes + l.stages * stage;
     l.bar_offset = l.bias_offset + bias;
     l.bytes = l.bar_offset + kBarBytes + 1024;
+    l.bytes = l.bytes < kTmemCtaMinSmem ? kTmemCtaMinSmem : l.bytes;  // (not at the sizes of today)
     return l;
 }
 

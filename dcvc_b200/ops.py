@@ -64,8 +64,9 @@ def conv1x1_f8(a, w, wscale, bias, epilogue=N.EPI_BIAS, out=None, block_n=0):
 
 
 def gemm_autotune(dtype, epilogue, M, Nn, K, sub_w=0, sub_cout=0):
-    """Times every valid N tile width of one conv1x1 shape on the current stream and records the
-    fastest for conv1x1(block_n=0) and the codecs.  Returns (block_n, microseconds per launch)."""
+    """Times every valid N tile width of one conv1x1 shape and the library's own choice on the current stream and
+    records the fastest width; conv1x1(block_n=0) and the codecs take it if it beat the library's choice.  Returns
+    (block_n, microseconds per launch)."""
     bn, us = ctypes.c_int(), ctypes.c_float()
     N.check(N.lib.dcvc_gemm_autotune(_DT[dtype], epilogue, M, Nn, K, sub_w, sub_cout, _stream(),
                                      ctypes.byref(bn), ctypes.byref(us)), "dcvc_gemm_autotune")
@@ -78,7 +79,7 @@ def gemm_autotune_enable(on=True):
 
 
 def gemm_tuned(dtype, epilogue, M, Nn, K, sub_w=0):
-    """The recorded tile width of a shape, 0 if it has not been tuned."""
+    """The recorded tile width of a shape, taken or not, 0 if it has not been tuned."""
     bn = ctypes.c_int()
     N.check(N.lib.dcvc_gemm_tuned(_DT[dtype], epilogue, M, Nn, K, sub_w, ctypes.byref(bn)),
             "dcvc_gemm_tuned")
